@@ -3,8 +3,8 @@
     python -m gpu_cdt_refine_b200.build
 
 libgqm_b200.so : refine.cu (kernels, driver, C ABI) + batch.cu (persistent
-                 batched engine, one-block small flip steps) + flipcl.cu
-                 (small flip steps on a thread-block cluster) + learned.cu (placement network training and
+                 batched engine) + flipcl.cu (the flip-flop loop in one
+                 cooperative launch) + learned.cu (placement network training and
                  inference) + cdt_gpu.cu (CDT construction on the GPU) +
                  legacy.cpp (C++ drop-in)
 libgqm_b200_fma.so : the same with GQM_CONTRACTED set: the products that the
@@ -75,8 +75,7 @@ def _cuda_jobs(force=False, extra=None, variant="separate"):
     units = {  # translation unit -> (the headers it includes, its own flags)
         "refine.cu": (hdr + refiner, []),
         "batch.cu": (hdr + refiner, []),
-        # phases on several SMs of a cluster: global loads are cached in L2 only
-        "flipcl.cu": (hdr + refiner, ["-Xptxas", "-dlcm=cg"]),
+        "flipcl.cu": (hdr + refiner, []),
         "learned.cu": (hdr + [os.path.join(CSRC, "learned.cuh")], []),
         "cdt_gpu.cu": ([os.path.join(INC, "gqm_cdt.h"), os.path.join(CSRC, "predicates.h"),
                         os.path.join(CSRC, "host_copy.h")], []),

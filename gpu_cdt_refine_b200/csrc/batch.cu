@@ -119,8 +119,16 @@ struct PPtLive {
   __device__ bool operator()(int i) const { return !(ps[i] & PS_DELETED); }
 };
 
-// launch timer that is never on (the block path is timed as a whole)
-__device__ KTimer g_ktimer_off;
+// The block as a team of flip_step.
+struct BlockTeam {
+  __device__ __forceinline__ int tid() const { return (int)threadIdx.x; }
+  __device__ __forceinline__ int size() const { return (int)blockDim.x; }
+  __device__ __forceinline__ bool lead() const { return threadIdx.x == 0; }
+  __device__ __forceinline__ bool sync() {
+    __syncthreads();
+    return true;
+  }
+};
 
 // ---------------------------------------------------------------------------
 // One domain of a batch, in device memory.  The host fills the inputs, the
@@ -179,9 +187,9 @@ __host__ __device__ inline Caps caps_of(int np, int nt, int ns) {
 // Scratch of one domain, carved from its block's arena.
 struct Scratch {
   Mesh M;
-  int *emptyt, *bad, *imark, *ilist, *sinks, *wl, *act, *win, *neg, *ll, *sl, *newidx, *tail;
-  int *emptyp, *pnew, *enclist, *encl2, *smark, *mids, *snap, *fq, *tl, *cav, *cavn;
-  uint8_t *clr;
+  int *emptyt, *bad, *imark, *ilist, *sinks, *wl, *newidx, *tail;
+  int *emptyp, *pnew, *enclist, *encl2, *smark, *mids, *snap, *cav, *cavn;
+  FlipLists fl;
   double2 *center;
   unsigned long long *hkeys;
   int *hvals, *s2ti;
@@ -214,30 +222,23 @@ __host__ __device__ inline void carve(Cursor &a, Scratch &S, const Caps &c) {
   M.tst = a.take<uint8_t>(T);
   M.tflip = a.take<uint8_t>(T);
   M.tfo = a.take<uint8_t>(T);
-  M.flip0 = a.take<uint8_t>(T);
-  S.clr = a.take<uint8_t>(T);
   M.tmark = a.take<int>(T);
-  M.tpos = a.take<int>(T);
   M.fstamp = a.take<int>(T);
-  M.tstamp = a.take<int>(T);
-  M.wbits = a.take<unsigned>(T / 32 + 1);
-  M.wcnt = a.take<int>(T / 1024 + 1);
-  M.wsup = a.take<int>(T / 32768 + 1);
-  M.wmeg = a.take<int>(T / 1048576 + 1);
   S.emptyt = a.take<int>(T);
   S.bad = a.take<int>(T);
   S.imark = a.take<int>(T);
   S.ilist = a.take<int>(T);
   S.sinks = a.take<int>(T);
   S.wl = a.take<int>(T);
-  S.act = a.take<int>(T);
-  S.win = a.take<int>(T);
-  S.neg = a.take<int>(T);
   S.newidx = a.take<int>(T);
-  S.fq = a.take<int>(T);
-  S.tl = a.take<int>(T);
-  S.ll = a.take<int>(2 * T);
-  S.sl = a.take<int>(6 * T);
+  M.fmark = a.take<unsigned long long>(T);
+  M.emap = a.take<int4>(T);
+  S.fl.q0 = a.take<int>(T);
+  S.fl.q1 = a.take<int>(T);
+  S.fl.rec = a.take<int4>(T);
+  S.fl.red = a.take<int>(2 * T);
+  S.fl.late = a.take<int4>(2 * Sg);
+  winner_carve(S.fl, a.take<unsigned>((long)winner_words(T)), T);
   S.center = a.take<double2>(T);
   M.s2t = a.take<s2t_t>(Sg);
   M.s2seg = a.take<int>(Sg);
@@ -376,44 +377,26 @@ struct Cta {
   __device__ const int *pslots() const { return sh.S.emptyp + (lenp - nempty_p); }
   __device__ const int *tslots() const { return sh.S.emptyt + (lent - nempty_t); }
 
-  // ---- flip-flop (refine.cu:2328-2490): the steps of refine.cu's flip graph ----
-  __device__ int flip_flop(int ntri) {
-    Scratch &S = sh.S;
+  // ---- flip-flop (refine.cu:2328-2490) ----
+  __device__ __noinline__ int flip_flop() {
+    const FlipLists &L = sh.S.fl;
     FlipCtl *fc = &sh.fc;
-    k_flip_entry_reset(S.M, ntri);
+    BlockTeam T;
+    FlipRegs R{fc->gen, fc->epoch, fc->steps};
+    const int entry = R.steps;
+    for (;;) {
+      const int n = vload(&fc->cnt.qn[R.gen & 1]);
+      if (n == 0) break;
+      if (flip_step<PRED>(sh.S.M, L, &fc->cnt, R, entry, T, (R.gen & 1) ? L.q1 : L.q0, n, L.rec, nullptr, nullptr) !=
+          FLIP_GO)
+        break;
+    }
     SYNC();
-    int n = compact(PNotNullFlag{S.M.tst, S.M.tflip}, Ident{}, 0, ntri, S.act);
     if (lead()) {
-      fc->nact = n;
-      fc->nact_next = 0;
-      fc->entry_steps = fc->steps;
-      flip_next(fc);
+      flip_close(fc, R);
+      fc->ran++;
     }
     SYNC();
-    while (fc->cond) {
-      FlipQ Q{S.fq, &fc->qn, &fc->gen};
-      TouchL T{S.tl, &fc->tn, &fc->gen};
-      k_check_flip2<PRED>(S.M, S.act, &fc->nact, S.clr, T, &g_ktimer_off);
-      SYNC();
-      k_flip_winner2(S.M, S.act, &fc->nact, S.clr, Q, S.win, &fc->winn);
-      SYNC();
-      k_link_phase1(S.M, S.win, &fc->winn, S.ll, S.sl, &fc->epoch);
-      SYNC();
-      k_phase2(S.M, S.win, &fc->winn, S.ll, S.sl);
-      SYNC();
-      k_phase3q(S.M, S.win, &fc->winn, S.sl, Q);
-      SYNC();
-      k_mark_red_steiner_q(S.M, S.tl, &fc->tn, Q);
-      SYNC();
-      k_flip_reset_filter(S.M, S.tl, &fc->tn, S.fq, &fc->qn, S.act, &fc->nact_next);
-      SYNC();
-      if (lead()) {
-        fc->nact = fc->nact_next;
-        fc->nact_next = 0;
-        flip_next(fc);
-      }
-      SYNC();
-    }
     return GQM_OK;  // errors raised on the device are read by the round loop
   }
 
@@ -435,9 +418,9 @@ struct Cta {
         if (ndel == 0) break;
         if (++inner > max_rounds) return GQM_ERR_ROUND_LIMIT;
         nmark = ndel;
-        k_mark_redundant(S.M, S.smark, S.mids, publish(C_LIST1, ndel));
+        k_mark_redundant(S.M, S.smark, S.mids, publish(C_LIST1, ndel), S.fl);
         SYNC();
-        int rc = flip_flop(last_triangle);
+        int rc = flip_flop();
         if (rc) return rc;
       }
       int rc = ensure_slots(nenc, 2 * nenc);
@@ -459,14 +442,14 @@ struct Cta {
         k_mid_snapshot(S.M, S.mids, dn, S.smark, S.snap);
         if (lead()) sh.fc.epoch++;
         SYNC();
-        k_insert_mid(S.M, S.mids, dn, S.smark, S.snap, pslots(), tslots(), last_subseg, &sh.fc.epoch, sh.ctr + 1);
+        k_insert_mid(S.M, S.mids, dn, S.smark, S.snap, pslots(), tslots(), last_subseg, S.fl, sh.ctr + 1);
         SYNC();
         k_update_mid_nbrs(S.M, S.mids, dn, S.smark, S.enclist);
         SYNC();
       }
       consume_slots(nenc, 2 * nenc);
       last_subseg += nenc;
-      rc = flip_flop(last_triangle);
+      rc = flip_flop();
       if (rc) return rc;
     }
     return GQM_OK;
@@ -507,12 +490,12 @@ struct Cta {
     k_reset_steiner(S.M, S.wl, dw, S.sinks);
     if (lead()) sh.fc.epoch++;
     SYNC();
-    k_insert_steiner(S.M, S.wl, dw, S.sinks, S.center, pslots(), tslots(), &sh.fc.epoch, sh.ctr + 0);
+    k_insert_steiner(S.M, S.wl, dw, S.sinks, S.center, pslots(), tslots(), S.fl, sh.ctr + 0);
     SYNC();
     k_update_steiner_nbrs(S.M, S.wl, dw, S.sinks);
     SYNC();
     consume_slots(nst, 2 * nst);
-    rc = flip_flop(last_triangle);
+    rc = flip_flop();
     if (rc) return rc;
     k_onsegs_to_enc(S.M, S.encl2, last_subseg);
     SYNC();
@@ -567,26 +550,17 @@ struct Cta {
       S.M.err = &sh.err;
       sh.err = 0;
       for (int i = 0; i < 6; ++i) sh.ctr[i] = 0;
-      FlipCtl &fc = sh.fc;
-      fc.gen = 0;
-      fc.epoch = 0;
-      fc.steps = 0;
-      fc.entry_steps = 0;
-      fc.cap_hit = 0;
-      fc.cond = 0;
-      fc.cap = 64 * max_rounds;
-      fc.errp = &sh.err;
-      for (int b = 0; b < kFlipProfileBins; ++b) fc.prof_steps[b] = fc.prof_items[b] = 0;
+      sh.fc.gen = 0;
+      sh.fc.epoch = 0;
+      ctl_reset(&sh.fc, 64 * max_rounds, &sh.err, true);
+      S.fl.c = &sh.fc;
     }
     SYNC();
-    // stamps, tags and winner counts start from zero for every domain
+    // stamps, claims and tags start afresh for every domain
     cta_fill(S.M.s2t, c.sphys, (s2t_t)0);
     cta_fill(S.M.fstamp, c.tphys, 0);
-    cta_fill(S.M.tstamp, c.tphys, 0);
-    cta_fill(S.M.wbits, c.tphys / 32 + 1, 0u);
-    cta_fill(S.M.wcnt, c.tphys / 1024 + 1, 0);
-    cta_fill(S.M.wsup, c.tphys / 32768 + 1, 0);
-    cta_fill(S.M.wmeg, c.tphys / 1048576 + 1, 0);
+    cta_fill(S.M.fmark, c.tphys, ~0ull);
+    cta_fill(S.M.emap, c.tphys, make_int4(0, 0, 0, 0));
     k_check_input(J.pts, np, J.tri, J.nbr, nt, reinterpret_cast<const int *>(J.seg), ns, &sh.err);
     k_goodcos(J.theta, sh.gc);
     SYNC();
@@ -659,7 +633,7 @@ struct Cta {
       if (rc == 0) {
         char *o = J.obase + J.ooff;
         k_emit_output(S.M, out_nt, last_subseg, reinterpret_cast<int *>(o + L.tri), reinterpret_cast<int *>(o + L.nbr),
-                      reinterpret_cast<int *>(o + L.seg), reinterpret_cast<uint8_t *>(o + L.ts));
+                      reinterpret_cast<int *>(o + L.seg), reinterpret_cast<uint8_t *>(o + L.ts), &sh.fc);
         k_emit_pstatus(S.M, out_np, reinterpret_cast<uint8_t *>(o + L.ps));
         double2 *op = reinterpret_cast<double2 *>(o + L.pts);
         for (int i = (int)threadIdx.x; i < out_np; i += (int)blockDim.x) op[i] = S.M.pts[i];
@@ -717,127 +691,7 @@ __global__ void __launch_bounds__(NT, MINB) k_batch(Job *jobs, const int *order,
     batch_body<0>(jobs, order, njobs, next, arenas, arena_stride, sh);
 }
 
-// ---------------------------------------------------------------------------
-// Small flip steps of the single-domain engine
-// ---------------------------------------------------------------------------
-// The single-domain flip-flop loop (refine.cu's flip graph: one launch per
-// step phase) spends most of its steps on small active sets: on the 2M-point
-// input three quarters of the steps have fewer than 2,048 triangles, where the
-// eight launches of a step cost more than the work.  This kernel runs in the
-// loop body after the step's condition kernel: while the next step's active
-// set has at most `limit` triangles, one block runs whole steps (the same
-// phases, compiled in block mode, separated by barriers), then it re-sets the
-// loop condition.  The steps and their results are the ones the grid kernels
-// would produce (every phase is decided by the reference's rules, not by the
-// thread layout).  The loop's control block (list lengths, stamps'
-// generation, launch epoch) is worked on in shared memory and written back
-// at exit: a step of a few triangles is a chain of dependent memory accesses,
-// and every counter read or atomic on shared memory instead of global memory
-// takes one L2 round trip out of that chain.
-constexpr int kSmallThreads = 512;
-template <int PRED>
-__global__ void __launch_bounds__(kSmallThreads, 1)
-    k_flip_small(Mesh M, FlipCtl *gfc, int *act, uint8_t *clr, int *win, int *ll, int *sl, int *fq, int *tl,
-                 int limit, cudaGraphConditionalHandle h, int graph, KTimer *tm) {
-  __shared__ int go;
-  __shared__ FlipCtl sfc;
-  FlipCtl *fc = &sfc;
-  if (threadIdx.x == 0) sfc = *gfc;
-  const int timed = tm->on;
-  const unsigned long long start = timed ? global_ns() : 0;
-  long long items = 0, wins = 0;  // thread 0's count of the launch's work (probe only)
-  for (;;) {
-    if (threadIdx.x == 0) go = fc->cond && fc->nact <= limit;
-    SYNC();
-    if (!go) break;
-    if (threadIdx.x == 0) items += fc->nact;
-    FlipQ Q{fq, &fc->qn, &fc->gen};
-    TouchL T{tl, &fc->tn, &fc->gen};
-    k_check_flip2<PRED>(M, act, &fc->nact, clr, T, &g_ktimer_off);
-    SYNC();
-    k_flip_winner2(M, act, &fc->nact, clr, Q, win, &fc->winn);
-    SYNC();
-    if (threadIdx.x == 0) wins += fc->winn;
-    k_link_phase1(M, win, &fc->winn, ll, sl, &fc->epoch);
-    SYNC();
-    k_phase2(M, win, &fc->winn, ll, sl);
-    SYNC();
-    k_phase3q(M, win, &fc->winn, sl, Q);
-    SYNC();
-    k_mark_red_steiner_q(M, tl, &fc->tn, Q);
-    SYNC();
-    k_flip_reset_filter(M, tl, &fc->tn, fq, &fc->qn, act, &fc->nact_next);
-    SYNC();
-    if (threadIdx.x == 0) {
-      fc->nact = fc->nact_next;
-      fc->nact_next = 0;
-      fc->small_steps++;
-      flip_next(fc);
-    }
-    SYNC();
-  }
-  if (threadIdx.x == 0) *gfc = sfc;
-#ifndef GQM_HOST_EMU
-  if (graph && threadIdx.x == 0) cudaGraphSetConditional(h, fc->cond);
-#endif
-  (void)h;
-  (void)graph;
-  if (timed) ktimer_end(tm, start, items, wins);
-}
-
 }  // namespace gqm
-
-// Launch of k_flip_small on the single-domain engine's buffers (refine.cu).
-// mesh points at the caller's Mesh (the same layout in both compilations);
-// timer is the caller's KTimer (the same layout too).
-int gqm_flip_small_launch(const void *mesh, size_t mesh_bytes, void *fc, int pred, int *act, uint8_t *clr, int *win,
-                          int *ll, int *sl, int *fq, int *tl, int limit, cudaStream_t st,
-                          cudaGraphConditionalHandle h, int graph, void *timer) {
-  if (mesh_bytes != sizeof(gqm::Mesh)) return GQM_ERR_ARGUMENT;
-  gqm::Mesh M;
-  memcpy(&M, mesh, sizeof(M));
-  gqm::FlipCtl *c = static_cast<gqm::FlipCtl *>(fc);
-  gqm::KTimer *tm = static_cast<gqm::KTimer *>(timer);
-#ifdef GQM_HOST_EMU
-  (void)st;
-  if (pred)
-    gqm::k_flip_small<1>(M, c, act, clr, win, ll, sl, fq, tl, limit, h, graph, tm);
-  else
-    gqm::k_flip_small<0>(M, c, act, clr, win, ll, sl, fq, tl, limit, h, graph, tm);
-#else
-  if (pred)
-    gqm::k_flip_small<1><<<1, gqm::kSmallThreads, 0, st>>>(M, c, act, clr, win, ll, sl, fq, tl, limit, h, graph, tm);
-  else
-    gqm::k_flip_small<0><<<1, gqm::kSmallThreads, 0, st>>>(M, c, act, clr, win, ll, sl, fq, tl, limit, h, graph, tm);
-#endif
-  return GQM_OK;
-}
-
-// The incircle expansion-fallback counter of this translation unit's kernels
-// (a device variable exists once per translation unit): added to *sum, then
-// zeroed when `reset` is set.  Called by the single-domain driver, which
-// reports the counters of all its kernels together.
-int gqm_fallbacks_cta(unsigned long long *sum, int reset, cudaStream_t st) {
-  unsigned long long v = 0;
-#ifdef GQM_HOST_EMU
-  (void)st;
-  v = gqm::g_incircle_fallbacks;
-  if (reset) gqm::g_incircle_fallbacks = 0;
-#else
-  if (cudaMemcpyFromSymbolAsync(&v, gqm::g_incircle_fallbacks, sizeof(v), 0, cudaMemcpyDeviceToHost, st) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return GQM_ERR_CUDA;
-  if (reset) {
-    const unsigned long long zero = 0;
-    if (cudaMemcpyToSymbolAsync(gqm::g_incircle_fallbacks, &zero, sizeof(zero), 0, cudaMemcpyHostToDevice, st) !=
-        cudaSuccess)
-      return GQM_ERR_CUDA;
-  }
-#endif
-  if (sum) *sum += v;
-  return GQM_OK;
-}
 
 // ===========================================================================
 // Host side

@@ -1,31 +1,30 @@
-// Small flip steps of the single-domain engine on one thread-block cluster.
+// The flip-flop loop of the single-domain engine in one launch.
 //
-// The flip-flop loop (GPU_Refine/refine.cu:2328-2490) spends most of its steps
-// on small active sets.  batch.cu's k_flip_small runs such steps in one thread
-// block; this kernel runs them on a cluster of 8 or 16 blocks (one per SM, up
-// to 4,096 threads), so that the items of a step are spread over more warps
-// and SMs while the step phases are still separated by a barrier instead of a
-// launch.  The phase functions are the kernels of kernels.cuh compiled in
-// cluster mode: each is a __device__ function whose grid-stride loop covers
-// the cluster (the launch's grid is exactly one cluster), and a cluster
-// barrier (release / acquire at cluster scope) separates consecutive phases.
+// flipFlop (GPU_Refine/refine.cu:2328-2490) runs a step after another until no
+// triangle is flagged.  Here the whole loop is one cooperative launch whose
+// blocks separate the phases of a step (flip_step in kernels.cuh) with a
+// barrier in global memory, and no launch, condition node or host read stands
+// between two phases or two steps.
 //
-// The phases communicate through global memory written by other SMs of the
-// cluster.  This translation unit is compiled with global loads cached in L2
-// only (ptxas -dlcm=cg), so no load can be served from a line that an SM's L1
-// kept from before the barrier; the barrier's release / acquire orders every
-// store before it with every load after it.
+// Most steps are small: of the ~1,030 steps of a 2,000,000-point refinement,
+// ~680 have at most 1,024 active triangles, and all blocks' barriers would
+// cost more than such a step's work.  Those steps are run by one team of the
+// first blocks while the others wait at one barrier: by default block 0 alone,
+// whose barrier is __syncthreads() and which keeps the list lengths, the queues
+// and the decisions in shared memory; gqm_tuning.small_cluster asks for 8 or 16
+// blocks instead.
 //
-// Every step makes the same decisions as the grid kernels and the one-block
-// kernel: each phase is decided by the reference's rules on the data, never by
-// the thread layout.
+// Threads: 512 per SM at up to 128 registers.  640, 768 and 1,024 threads (96,
+// 80 and 64 registers) gave 72.5, 72.7 and 75.2 ms for the refinement of
+// 2,000,000 points against 71.2 ms: more warps do not shorten the chains.
+//
+// Every wait is bounded; one that runs out records GQM_ERR_TOPOLOGY and every
+// block leaves the loop.
 #define GQM_CLUSTER_MODE 1
 #define gqm gqm_cl
 #include <cuda_runtime.h>
-#ifndef GQM_HOST_EMU
-#include <cooperative_groups.h>
-#endif
 
+#include <chrono>
 #include <cstring>
 
 #include "../../include/gqm_refine.h"
@@ -33,140 +32,228 @@
 
 namespace gqm {
 
-__device__ KTimer g_ktimer_cluster_off;
+// One thread block.
+struct BlockTeam {
+  __device__ __forceinline__ int tid() const { return (int)threadIdx.x; }
+  __device__ __forceinline__ int size() const { return (int)blockDim.x; }
+  __device__ __forceinline__ bool lead() const { return threadIdx.x == 0; }
+  __device__ __forceinline__ bool sync() {
+    __syncthreads();
+    return true;
+  }
+};
 
-// threads per block of the cluster kernel; one block per SM
-constexpr int kClusterThreads = 256;
-
-__device__ __forceinline__ void cluster_barrier() {
-#ifndef GQM_HOST_EMU
-  cooperative_groups::this_cluster().sync();
+// The first `nb` blocks of the launch.  A barrier adds one arrival per block to
+// a word that only grows (it starts at zero with every refinement); a block
+// waits until all arrivals of its own barrier have been counted.  The arrival
+// is a reduction with no answer to wait for, and the wait polls one word.
+struct GridBar {
+  unsigned long long arrived;  // arrivals of all barriers
+  unsigned long long base;     // arrivals when the current launch began
+  int broken;
+};
+constexpr unsigned kBarrierPolls = 1u << 25;  // tens of seconds
+struct GridTeam {
+  GridBar *bar;
+  int nb;
+  unsigned long long target;
+  int *err;
+  __device__ __forceinline__ int tid() const { return (int)(blockIdx.x * blockDim.x + threadIdx.x); }
+  __device__ __forceinline__ int size() const { return nb * (int)blockDim.x; }
+  __device__ __forceinline__ bool lead() const { return blockIdx.x == 0 && threadIdx.x == 0; }
+  __device__ __forceinline__ bool sync() {
+#ifdef GQM_HOST_EMU
+    return true;
+#else
+    target += (unsigned long long)nb;
+    __syncthreads();
+    int ok = 1;
+    if (threadIdx.x == 0) {
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+      asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(&bar->arrived), "l"(1ull) : "memory");
+      unsigned polls = 0;
+      unsigned long long v;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(&bar->arrived) : "memory");
+        if (v >= target) break;
+        if (++polls > 64u) __nanosleep(64);
+        if (polls >= kBarrierPolls || ((polls & 1023u) == 0 && *(volatile int *)&bar->broken)) {
+          *(volatile int *)&bar->broken = 1;
+          atomicCAS(err, 0, GQM_ERR_TOPOLOGY);
+          ok = 0;
+          break;
+        }
+      }
+      asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    }
+    return __syncthreads_and(threadIdx.x == 0 ? ok : 1) != 0;
 #endif
+  }
+};
+
+// shared-memory copies of the small steps' lists
+constexpr int kSmallCap = 1024;
+struct SmallLists {
+  FlipCnt cnt;
+  int4 rec[kSmallCap];
+};
+
+template <int PRED, int NT>
+__global__ void __launch_bounds__(NT, 1)
+    k_flip_loop(Mesh mesh, FlipLists lists, GridBar *bars, const int *team, int small_limit, int small_team,
+                KTimer *ktm, KTimer *stm) {
+  const int nb = min(*team, (int)gridDim.x);  // blocks this refinement uses; the rest leave at once
+  if ((int)blockIdx.x >= nb) return;
+  __shared__ SmallLists sh;
+  __shared__ Mesh M;  // the phases are calls: they read the pointers from shared memory
+  __shared__ FlipLists L;
+  if (threadIdx.x == 0) {
+    M = mesh;
+    L = lists;
+  }
+  __syncthreads();
+  FlipCtl *c = lists.c;
+  FlipRegs R{c->gen, c->epoch, c->steps};
+  const int entry = R.steps;
+  const int st_blocks = min(small_team, nb);
+  GridTeam G{bars, nb, bars[0].base, c->errp};
+  GridTeam S{bars + 1, st_blocks, bars[1].base, c->errp};
+  const int timed = ktm->on;
+  const unsigned long long t0 = G.lead() ? global_ns() : 0;
+  int status = FLIP_GO;
+  // Every block takes the same way through the loop: what it decides on (list
+  // lengths, the control block) was written before the last barrier of all
+  // blocks and is not written again before the next.
+  while (status == FLIP_GO) {
+    const int n = vload(&c->cnt.qn[R.gen & 1]);
+    if (n == 0) break;
+    if (n > small_limit) {
+      status = flip_step<PRED>(M, L, &c->cnt, R, entry, G, (R.gen & 1) ? L.q1 : L.q0, n, L.rec, timed ? ktm : nullptr,
+                               nullptr);
+      continue;
+    }
+    // small steps
+    const int steps0 = R.steps;
+    if ((int)blockIdx.x < st_blocks) {
+      const unsigned long long s0 = timed && G.lead() ? global_ns() : 0;
+      int items = 0, wins = 0, m = n;
+      if (st_blocks == 1) {
+        BlockTeam B;
+        if (B.lead()) sh.cnt = c->cnt;
+        B.sync();
+        while (status == FLIP_GO && m > 0 && m <= small_limit) {
+          items += m;
+          status = flip_step<PRED>(M, L, &sh.cnt, R, entry, B, (R.gen & 1) ? L.q1 : L.q0, m,
+                                   m <= kSmallCap ? sh.rec : L.rec, nullptr, timed ? &wins : nullptr);
+          m = vload(&sh.cnt.qn[R.gen & 1]);
+        }
+        B.sync();
+        if (B.lead()) c->cnt = sh.cnt;
+      } else {
+        while (status == FLIP_GO && m > 0 && m <= small_limit) {
+          items += m;
+          status = flip_step<PRED>(M, L, &c->cnt, R, entry, S, (R.gen & 1) ? L.q1 : L.q0, m, L.rec, nullptr,
+                                   timed ? &wins : nullptr);
+          m = vload(&c->cnt.qn[R.gen & 1]);
+        }
+      }
+      if (G.lead()) {
+        c->gen = R.gen;
+        c->epoch = R.epoch;
+        c->steps = R.steps;
+        c->small_steps += R.steps - steps0;
+        L.c->small_status = status;
+        if (timed) ktimer_add(stm, s0, items, wins);
+      }
+    }
+    if (!G.sync()) {
+      status = FLIP_BROKEN;
+      break;
+    }
+    R.gen = vload(&c->gen);
+    R.epoch = (unsigned)vload((const int *)&c->epoch);
+    R.steps = vload(&c->steps);
+    status = vload(&c->small_status);
+  }
+  if (status != FLIP_BROKEN && !G.sync()) status = FLIP_BROKEN;  // nobody reads the control block any more
+  if (G.lead()) {
+    flip_close(c, R);
+    c->ran++;
+    c->loop_ns += global_ns() - t0;
+    c->loops++;
+    if (status != FLIP_BROKEN) {
+      bars[0].base = G.target;
+      bars[1].base = bars[1].arrived;
+    }
+  }
 }
 
-template <int PRED>
-__global__ void __launch_bounds__(kClusterThreads, 1)
-    k_flip_small_cl(Mesh M, FlipCtl *fc, int *act, uint8_t *clr, int *win, int *ll, int *sl, int *fq, int *tl,
-                    int limit, cudaGraphConditionalHandle h, int graph, KTimer *tm) {
-  const int timed = tm->on;
-  const unsigned long long start = timed ? global_ns() : 0;
-  long long items = 0, wins = 0;  // the launch's work, the same in every thread (probe only)
-  for (;;) {
-    // Every thread reads the same two words: they were last written before
-    // the barrier that ended the previous step (or by the kernel before this
-    // launch), and nothing writes them until after the next barrier.
-    const int nact = fc->nact;
-    const int go = fc->cond && nact <= limit;
-    cluster_barrier();
-    if (!go) break;
-    items += nact;
-    FlipQ Q{fq, &fc->qn, &fc->gen};
-    TouchL T{tl, &fc->tn, &fc->gen};
-    k_check_flip2<PRED>(M, act, &fc->nact, clr, T, &g_ktimer_cluster_off);
-    cluster_barrier();
-    k_flip_winner2(M, act, &fc->nact, clr, Q, win, &fc->winn);
-    cluster_barrier();
-    wins += fc->winn;  // complete after the barrier; read before the next step resets it
-    k_link_phase1(M, win, &fc->winn, ll, sl, &fc->epoch);
-    cluster_barrier();
-    k_phase2(M, win, &fc->winn, ll, sl);
-    cluster_barrier();
-    k_phase3q(M, win, &fc->winn, sl, Q);
-    cluster_barrier();
-    k_mark_red_steiner_q(M, tl, &fc->tn, Q);
-    cluster_barrier();
-    k_flip_reset_filter(M, tl, &fc->tn, fq, &fc->qn, act, &fc->nact_next);
-    cluster_barrier();
-    if (GQM_BLOCK0 && threadIdx.x == 0) {
-      fc->nact = fc->nact_next;
-      fc->nact_next = 0;
-      fc->small_steps++;
-      flip_next(fc);
-    }
-    cluster_barrier();
-  }
-#ifndef GQM_HOST_EMU
-  if (graph && GQM_BLOCK0 && threadIdx.x == 0) cudaGraphSetConditional(h, fc->cond);
-#endif
-  (void)h;
-  (void)graph;
-  if (timed) ktimer_end(tm, start, items, wins);
+constexpr int kLoopThreads[2] = {256, 512};  // one block per SM at up to 255 / 128 registers
+typedef void (*LoopFn)(Mesh, FlipLists, GridBar *, const int *, int, int, KTimer *, KTimer *);
+static LoopFn loop_fn(int pred, int budget) {
+  if (budget == 1) return pred ? k_flip_loop<1, 256> : k_flip_loop<0, 256>;
+  return pred ? k_flip_loop<1, 512> : k_flip_loop<0, 512>;
 }
 
 }  // namespace gqm
 
-// Whether a cluster of `csize` blocks of the small-step kernel can be resident
-// on the current device (csize 8 or 16).  16 is beyond the portable cluster
-// size and is allowed explicitly.
-int gqm_flip_cluster_ok(int csize) {
+// Bytes of the barrier words that gqm_flip_loop_launch needs (zeroed before
+// every refinement).
+size_t gqm_flip_bar_bytes() { return 2 * sizeof(gqm::GridBar); }
+
+// Most blocks of a launch that can be resident together, one per SM.
+int gqm_flip_max_blocks(int budget) {
 #ifdef GQM_HOST_EMU
-  return csize == 8 || csize == 16;
+  (void)budget;
+  return 1;
 #else
-  if (csize != 8 && csize != 16) return 0;
-  int n0 = 0, n1 = 0;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
   for (int pred = 0; pred < 2; ++pred) {
-    const void *fn = pred ? (const void *)gqm::k_flip_small_cl<1> : (const void *)gqm::k_flip_small_cl<0>;
-    if (csize > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-      cudaGetLastError();
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)gqm::loop_fn(pred, budget),
+                                                      gqm::kLoopThreads[budget == 1 ? 0 : 1], 0) != cudaSuccess ||
+        per < 1)
       return 0;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)csize;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)csize);
-    cfg.blockDim = dim3(gqm::kClusterThreads);
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    (pred ? n1 : n0) = clusters;
   }
-  return n0 > 0 && n1 > 0;
+  return sms;
 #endif
 }
 
-// Launch of k_flip_small_cl on the single-domain engine's buffers (refine.cu):
-// one cluster of `csize` blocks.  mesh points at the caller's Mesh (the same
-// layout in every compilation).
-int gqm_flip_small_cl_launch(const void *mesh, size_t mesh_bytes, void *fc, int pred, int *act, uint8_t *clr,
-                             int *win, int *ll, int *sl, int *fq, int *tl, int limit, int csize, cudaStream_t st,
-                             cudaGraphConditionalHandle h, int graph, void *timer) {
-  if (mesh_bytes != sizeof(gqm::Mesh) || (csize != 8 && csize != 16)) return GQM_ERR_ARGUMENT;
+// Launch of k_flip_loop on the single-domain engine's buffers (refine.cu).
+// mesh and lists point at the caller's Mesh and FlipLists (the same layouts in
+// every compilation); *team is the number of blocks the refinement uses.
+int gqm_flip_loop_launch(const void *mesh, size_t mesh_bytes, const void *lists, size_t lists_bytes, void *bars,
+                         const int *team, int pred, int blocks, int budget, int small_limit, int small_team,
+                         void *ktimer, void *stimer, cudaStream_t st) {
+  if (mesh_bytes != sizeof(gqm::Mesh) || lists_bytes != sizeof(gqm::FlipLists)) return GQM_ERR_ARGUMENT;
   gqm::Mesh M;
+  gqm::FlipLists L;
   memcpy(&M, mesh, sizeof(M));
-  gqm::FlipCtl *c = static_cast<gqm::FlipCtl *>(fc);
-  gqm::KTimer *tm = static_cast<gqm::KTimer *>(timer);
+  memcpy(&L, lists, sizeof(L));
+  gqm::GridBar *b = static_cast<gqm::GridBar *>(bars);
+  gqm::KTimer *kt = static_cast<gqm::KTimer *>(ktimer), *stm = static_cast<gqm::KTimer *>(stimer);
 #ifdef GQM_HOST_EMU
+  (void)blocks;
   (void)st;
-  if (pred)
-    gqm::k_flip_small_cl<1>(M, c, act, clr, win, ll, sl, fq, tl, limit, h, graph, tm);
-  else
-    gqm::k_flip_small_cl<0>(M, c, act, clr, win, ll, sl, fq, tl, limit, h, graph, tm);
+  gqm::loop_fn(pred, budget)(M, L, b, team, small_limit, small_team, kt, stm);
   return GQM_OK;
 #else
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = (unsigned)csize;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)csize);
-  cfg.blockDim = dim3(gqm::kClusterThreads);
-  cfg.dynamicSmemBytes = 0;
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)gqm::kLoopThreads[budget == 1 ? 0 : 1]);
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaError_t e = pred ? cudaLaunchKernelEx(&cfg, gqm::k_flip_small_cl<1>, M, c, act, clr, win, ll, sl, fq, tl,
-                                            limit, h, graph, tm)
-                       : cudaLaunchKernelEx(&cfg, gqm::k_flip_small_cl<0>, M, c, act, clr, win, ll, sl, fq, tl,
-                                            limit, h, graph, tm);
-  return e == cudaSuccess ? GQM_OK : GQM_ERR_CUDA;
+  return cudaLaunchKernelEx(&cfg, gqm::loop_fn(pred, budget), M, L, b, team, small_limit, small_team, kt, stm) ==
+                 cudaSuccess
+             ? GQM_OK
+             : GQM_ERR_CUDA;
 #endif
 }
 
@@ -181,9 +268,9 @@ int gqm_fallbacks_cluster(unsigned long long *sum, int reset, cudaStream_t st) {
   v = gqm::g_incircle_fallbacks;
   if (reset) gqm::g_incircle_fallbacks = 0;
 #else
-  if (cudaMemcpyFromSymbolAsync(&v, gqm::g_incircle_fallbacks, sizeof(v), 0, cudaMemcpyDeviceToHost, st) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
+  if (sum && (cudaMemcpyFromSymbolAsync(&v, gqm::g_incircle_fallbacks, sizeof(v), 0, cudaMemcpyDeviceToHost, st) !=
+                  cudaSuccess ||
+              cudaStreamSynchronize(st) != cudaSuccess))
     return GQM_ERR_CUDA;
   if (reset) {
     const unsigned long long zero = 0;

@@ -10,13 +10,13 @@
 //   tst   uint8[Tcap]     NOTNULL | BAD | CHECK
 //   tflip uint8[Tcap]     flip-flop marker (set concurrently)
 //   tfo   uint8[Tcap]     flip orientation code, 15 = none
-//   tmark int[Tcap]       ownership marker (atomicMin) / flipBy
+//   tmark int[Tcap]       ownership marker of insertions (atomicMin)
+//   fmark uint64[Tcap]    claim of a flip step (atomicMin), fstamp int[Tcap]
+//   emap  int4[Tcap]      edge map of a flip step
 //   s2t   u128[Scap]      subsegment -> oriented triangle in the low word,
 //                         tagged with the launch epoch and the storing
 //                         thread's key (see s2t_store)
 //   s2seg int[Scap], enc int[Scap], segs int2[S_in]
-//   wbits uint32[Tcap/2^5], wcnt int[Tcap/2^10], wsup int[Tcap/2^15],
-//   wmeg int[Tcap/2^20]   flip winners of a step (bitmap and counts)
 // Edge i of a triangle joins vertices i+1 and i+2 and faces vertex i; an
 // oriented triangle (t << 2 | i) names edge i of t (GPU_Refine/refine.cu:95-113).
 // Flags the reference keeps in one byte (GPU_Refine/refine.h:36-205) are split
@@ -40,15 +40,12 @@ struct Mesh {
   double2 *pts;
   uint8_t *ps, *pred;
   int4 *tv, *tn, *tsg;
-  uint8_t *tst, *tflip, *tfo, *flip0;
+  uint8_t *tst, *tflip, *tfo;
   int *tmark;
-  int *tpos;  // winner-slot of each triangle during a flip step
-  int *fstamp, *tstamp;  // per-triangle generation stamps deduplicating the flip-step queues
+  int *fstamp;  // generation that last queued the triangle for a flip step
+  unsigned long long *fmark;  // claim of a flip step (see claim_key)
+  int4 *emap;  // where the triangle's edges went in the flip step of generation w
   s2t_t *s2t;
-  // flip winners of the current step: one bit per triangle slot and winner
-  // counts per 2^10, 2^15 and 2^20 slots (see win_rank)
-  unsigned *wbits;
-  int *wcnt, *wsup, *wmeg;
   int *s2seg, *enc;
   const int2 *segs;
   int *err;  // first error code raised on the device
@@ -102,31 +99,11 @@ __device__ __forceinline__ void s2t_store(const Mesh &M, int s, int v, uint32_t 
   }
 }
 
-// Position of flip winner `index` in the reference's winner list, which is
-// compacted in triangle order (kernelUpdatePhase1's pos, refine.cu:1312): the
-// number of this step's winners with a smaller slot.  The winners' own list
-// here is filled by atomics in any order, so the position is counted from the
-// winner bitmap and its counts per 2^10, 2^15 and 2^20 slots: at most 31
-// entries of each level (one 128-byte line each) plus the 2^20 counts before
-// the slot, all independent loads.  Only stores into subseg2tri need it.
-__device__ __forceinline__ int sum32(const int *a, int lo, int hi) {  // a[lo..hi), hi - lo < 32
-  int r = 0;
-#pragma unroll
-  for (int j = 0; j < 31; ++j)
-    if (lo + j < hi) r += a[lo + j];
-  return r;
+// A store that no other thread of the launch competes with.
+__device__ __forceinline__ void s2t_put(const Mesh &M, int s, int v, uint32_t epoch) {
+  M.s2t[s] = ((s2t_t)epoch << 64) | ((s2t_t)0xFFFFFFFFu << 32) | (uint32_t)v;
 }
-__device__ __forceinline__ int win_rank(const Mesh &M, int index) {
-  const int w = index >> 5, c = index >> 10, sc = index >> 15, mg = index >> 20;
-  int r = 0;
-  for (int i = 0; i < mg; ++i) r += M.wmeg[i];
-  r += sum32(M.wsup, mg << 5, sc) + sum32(M.wcnt, sc << 5, c);
-  int b = 0;
-#pragma unroll
-  for (int j = 0; j < 31; ++j)
-    if ((c << 5) + j < w) b += __popc(M.wbits[(c << 5) + j]);
-  return r + b + __popc(M.wbits[w] & ((1u << (index & 31)) - 1u));
-}
+
 // Slot in a list whose length *n many threads bump at once: the lanes of a
 // warp that arrive together take consecutive slots with one atomic, issued by
 // the lowest of them, instead of one atomic each on the same word.  The order
@@ -143,6 +120,19 @@ __device__ __forceinline__ int list_slot(int *n) {
   return base + __popc(m & ((1u << lane) - 1u));
 #endif
 }
+// Two consecutive slots.
+__device__ __forceinline__ int list_slot2(int *n) {
+#ifdef GQM_HOST_EMU
+  return atomicAdd(n, 2);
+#else
+  const unsigned m = __activemask();
+  const int lane = (int)(threadIdx.x & 31u), leader = __ffs(m) - 1;
+  int base = 0;
+  if (lane == leader) base = atomicAdd(n, 2 * __popc(m));
+  base = __shfl_sync(m, base, leader);
+  return base + 2 * __popc(m & ((1u << lane) - 1u));
+#endif
+}
 // The same for an event counter: one atomic per warp.
 __device__ __forceinline__ void count_event(unsigned long long *c) {
 #ifdef GQM_HOST_EMU
@@ -152,37 +142,6 @@ __device__ __forceinline__ void count_event(unsigned long long *c) {
   if ((int)(threadIdx.x & 31u) == __ffs(m) - 1) atomicAdd(c, (unsigned long long)__popc(m));
 #endif
 }
-// enter / leave the winner bitmap and its counts.  The two coarse counts
-// (2^15 and 2^20 slots) are few and hot, so the lanes of a warp that hit the
-// same one add together (one atomic per distinct counter); `on` says whether
-// this lane takes part (every lane of the warp must call).
-__device__ __forceinline__ void win_count(int *a, int idx, bool on, int d) {
-#ifdef GQM_HOST_EMU
-  if (on) atomicAdd(a + idx, d);
-#else
-  const unsigned act = __ballot_sync(0xffffffffu, on);
-  if (!on) return;
-  const unsigned same = __match_any_sync(act, idx);
-  if ((int)(threadIdx.x & 31u) == __ffs(same) - 1) atomicAdd(a + idx, d * __popc(same));
-#endif
-}
-__device__ __forceinline__ void win_mark(const Mesh &M, int index, bool on) {
-  if (on) {
-    atomicOr(M.wbits + (index >> 5), 1u << (index & 31));
-    atomicAdd(M.wcnt + (index >> 10), 1);
-  }
-  win_count(M.wsup, on ? index >> 15 : -1, on, 1);
-  win_count(M.wmeg, on ? index >> 20 : -1, on, 1);
-}
-__device__ __forceinline__ void win_unmark(const Mesh &M, int index, bool on) {
-  if (on) {
-    atomicAnd(M.wbits + (index >> 5), ~(1u << (index & 31)));
-    atomicAdd(M.wcnt + (index >> 10), -1);
-  }
-  win_count(M.wsup, on ? index >> 15 : -1, on, -1);
-  win_count(M.wmeg, on ? index >> 20 : -1, on, -1);
-}
-
 __device__ __forceinline__ void raise_err(const Mesh &M, int code) { atomicCAS(M.err, 0, code); }
 
 // ---------------------------------------------------------------------------
@@ -206,12 +165,13 @@ __device__ __noinline__ double incircle_slow(double2 a, double2 b, double2 c, do
   if (PRED == 0) return gqm_incircle_zero_fallback_ref(a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y);
   return gqm_incircle_exact(a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y);
 }
+// The test before any fallback; *open is set when its sign is not decided.
 template <int PRED>
-__device__ __forceinline__ double incircle(double2 a, double2 b, double2 c, double2 d) {
+__device__ __forceinline__ double incircle_fast(double2 a, double2 b, double2 c, double2 d, bool *open) {
   if (PRED == 0) {
-    double r = gqm_incircle_det_ref(a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y);
-    if (r != 0) return r;
-    return incircle_slow<0>(a, b, c, d);
+    const double r = gqm_incircle_det_ref(a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y);
+    if (r == 0) *open = true;
+    return r;
   }
   // exact: filter then exact expansion
   double adx = a.x - d.x, bdx = b.x - d.x, cdx = c.x - d.x;
@@ -223,8 +183,14 @@ __device__ __forceinline__ double incircle(double2 a, double2 b, double2 c, doub
   double perm = (fabs(bdxcdy) + fabs(cdxbdy)) * alift + (fabs(cdxady) + fabs(adxcdy)) * blift +
                 (fabs(adxbdy) + fabs(bdxady)) * clift;
   double eb = (10.0 + 96.0 * GQM_EPS) * GQM_EPS * perm;
-  if (det > eb || -det > eb) return det;
-  return incircle_slow<1>(a, b, c, d);
+  if (!(det > eb || -det > eb)) *open = true;
+  return det;
+}
+template <int PRED>
+__device__ __forceinline__ double incircle(double2 a, double2 b, double2 c, double2 d) {
+  bool open = false;
+  const double r = incircle_fast<PRED>(a, b, c, d, &open);
+  return open ? incircle_slow<PRED>(a, b, c, d) : r;
 }
 
 // checkseg4encroach, GPU_Refine/refine.cu:115-139 (goodcoss squared once).

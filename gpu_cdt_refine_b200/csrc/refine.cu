@@ -44,17 +44,13 @@ struct NvtxRange {
 };
 #endif
 
-// batch.cu: the flip steps of small active sets in one block
-int gqm_flip_small_launch(const void *mesh, size_t mesh_bytes, void *fc, int pred, int *act, uint8_t *clr, int *win,
-                          int *ll, int *sl, int *fq, int *tl, int limit, cudaStream_t st,
-                          cudaGraphConditionalHandle h, int graph, void *timer);
-// flipcl.cu: the same on one thread-block cluster of csize blocks
-int gqm_flip_small_cl_launch(const void *mesh, size_t mesh_bytes, void *fc, int pred, int *act, uint8_t *clr,
-                             int *win, int *ll, int *sl, int *fq, int *tl, int limit, int csize, cudaStream_t st,
-                             cudaGraphConditionalHandle h, int graph, void *timer);
-int gqm_flip_cluster_ok(int csize);
-// the incircle expansion-fallback counters of batch.cu's and flipcl.cu's kernels
-int gqm_fallbacks_cta(unsigned long long *sum, int reset, cudaStream_t st);
+// flipcl.cu: the flip-flop loop in one cooperative launch
+size_t gqm_flip_bar_bytes();
+int gqm_flip_max_blocks(int budget);
+int gqm_flip_loop_launch(const void *mesh, size_t mesh_bytes, const void *lists, size_t lists_bytes, void *bars,
+                         const int *team, int pred, int blocks, int budget, int small_limit, int small_team,
+                         void *ktimer, void *stimer, cudaStream_t st);
+// the incircle expansion-fallback counter of flipcl.cu's kernels
 int gqm_fallbacks_cluster(unsigned long long *sum, int reset, cudaStream_t st);
 
 namespace gqm {
@@ -237,18 +233,6 @@ struct ValueOf {
   const int *a;
   __device__ int operator()(int i) const { return a[i]; }
 };
-struct PNotNullFlag {
-  const uint8_t *tst, *flag;
-  __device__ bool operator()(int i) const { return (tst[i] & TS_NOTNULL) && flag[i]; }
-};
-struct PWinner {
-  const uint8_t *tst, *tfo;
-  __device__ bool operator()(int i) const { return (tst[i] & TS_NOTNULL) && tfo[i] != 15; }
-};
-struct PNeg {
-  const int *a;
-  __device__ bool operator()(int i) const { return a[i] < 0; }
-};
 struct PNonNeg {
   const int *a;
   __device__ bool operator()(int i) const { return a[i] >= 0; }
@@ -302,6 +286,7 @@ struct DState {
   int pslot, tslot;  // first free slot of the current batch: lenp - nempty_p, lent - nempty_t
   int req_p, req_t, grew;  // the batch's request; whether a growth step happened
   int nenc, nmark, ndel, nmid, nbad, nst;
+  int team;  // blocks of the flip loop's launch that this refinement uses
   // a physical capacity would be exceeded (1 points, 2 triangles, 4
   // subsegments, 8 stored cavities): every loop ends and the host repeats the
   // run with larger buffers (the result does not depend on them)
@@ -648,16 +633,16 @@ struct Refiner {
   int pointblock = 0, triblock = 0;
   // per-triangle scratch (capacity tphys)
   int *emptyt = nullptr, *bad = nullptr, *imark = nullptr, *ilist = nullptr, *sinks = nullptr, *wl = nullptr;
-  int *act = nullptr, *win = nullptr, *neg = nullptr, *ll = nullptr, *sl = nullptr, *newidx = nullptr;
+  int *newidx = nullptr;
   int *tail = nullptr;
   double2 *center = nullptr;
   int *cav = nullptr, *cavn = nullptr;  // stored cavities of the Steiner candidates
   long cav_cap = 0;
-  int *fq = nullptr, *tl = nullptr;  // flip-step queue and claimed-triangle list
-  uint8_t *clr = nullptr;            // deferred flag clears of a flip step
-  FlipCtl *fc = nullptr;             // flip-loop control block (device)
-  KTimer *ktm = nullptr;             // launch timer of the flip-step check kernel
-  KTimer *stm = nullptr;             // launch timer of the small-step kernel
+  FlipLists fl{};         // lists of the flip steps, and their control block (device)
+  FlipCtl *fc = nullptr;  // = fl.c
+  char *bars = nullptr;   // barrier words of the flip loop's launch
+  KTimer *ktm = nullptr;  // timer of the check phase of the steps run by all blocks
+  KTimer *stm = nullptr;  // timer of the small steps
   // the driver's state on the device, and the refinement captured as one
   // CUDA graph (loops and branches as conditional nodes)
   DState *ds = nullptr;
@@ -767,20 +752,19 @@ struct Refiner {
 
   void release() {
     drop_ref_graph();
-    void *ptrs[] = {M.pts, M.ps, M.pred, M.tv, M.tn, M.tsg, M.tst, M.tflip, M.tfo, M.flip0, M.tmark, M.tpos,
-                    M.s2t, M.s2seg, M.enc, M.err, stm, emptyt, bad, imark, ilist, sinks, wl, act, win, neg, ll, sl,
+    void *ptrs[] = {M.pts, M.ps, M.pred, M.tv, M.tn, M.tsg, M.tst, M.tflip, M.tfo, M.tmark, M.fmark, M.emap,
+                    M.s2t, M.s2seg, M.enc, M.err, stm, emptyt, bad, imark, ilist, sinks, wl,
                     newidx, tail, center, emptyp, pnew, enclist, encl2, smark, mids, snap, segs, dcount, bc,
-                    dctr, dgc, dinput, mlp_w, mlp_b, M.fstamp, M.tstamp, fq, tl, clr, fc, cav, cavn, ktm, M.wbits, M.wcnt, M.wsup, M.wmeg,
-                    ds, csync};
+                    dctr, dgc, dinput, mlp_w, mlp_b, M.fstamp, fl.q0, fl.q1, fl.rec, fl.red, fl.late, fl.wbits, fc, cav, cavn, ktm, bars, ds, csync};
     for (void *p : ptrs)
       if (p) cudaFree(p);
     if (hcount) cudaFreeHost(hcount);
     hcount = nullptr;
     M = Mesh{};
-    emptyt = bad = imark = ilist = sinks = wl = act = win = neg = ll = sl = newidx = tail = nullptr;
-    fq = tl = nullptr;
-    clr = nullptr;
+    emptyt = bad = imark = ilist = sinks = wl = newidx = tail = nullptr;
+    fl = FlipLists{};
     fc = nullptr;
+    bars = nullptr;
     ktm = nullptr;
     stm = nullptr;
     mlp_w = nullptr;
@@ -822,11 +806,14 @@ struct Refiner {
     if (!st && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GQM_ERR_CUDA;
     if (!ev0) cudaEventCreate(&ev0);
     if (!ev1) cudaEventCreate(&ev1);
+    for (int b = 1; b <= 2; ++b)
+      if (loop_blocks[b] <= 0 && (loop_blocks[b] = gqm_flip_max_blocks(b)) <= 0) return GQM_ERR_CUDA;
     if (!dcount) {
       if (dalloc(&dcount, 16) || dalloc(&bc, kMaxCompactBlocks + 1) || dalloc(&dctr, 8) || dalloc(&dgc, 2) ||
           dalloc(&M.err, 1) || dalloc(&fc, 1) || dalloc(&ktm, 1) || dalloc(&stm, 1) || dalloc(&ds, 1) ||
-          dalloc(&csync, 1))
+          dalloc(&csync, 1) || dalloc(&bars, gqm_flip_bar_bytes()))
         return GQM_ERR_MEMORY;
+      fl.c = fc;
       cudaMemsetAsync(csync, 0, sizeof(CompactSync), st);
       cudaMemsetAsync(fc, 0, sizeof(FlipCtl), st);
       cudaMemsetAsync(ktm, 0, sizeof(KTimer), st);  // off until gqm_context_probe
@@ -930,29 +917,22 @@ struct Refiner {
     long old = tphys;
     if (n <= old) return GQM_OK;
     if (regrow(&M.tv, old, n) || regrow(&M.tn, old, n) || regrow(&M.tsg, old, n) || regrow(&M.tst, old, n) ||
-        regrow(&M.tflip, old, n) || regrow(&M.tfo, old, n) || regrow(&M.flip0, old, n) ||
-        regrow(&M.tmark, old, n) || regrow(&M.tpos, old, n) || regrow(&emptyt, 0, n) || regrow(&bad, old, n) ||
+        regrow(&M.tflip, old, n) || regrow(&M.tfo, old, n) || regrow(&M.tmark, old, n) ||
+        regrow(&M.fmark, old, n) || regrow(&M.emap, old, n) || regrow(&emptyt, 0, n) || regrow(&bad, old, n) ||
         regrow(&imark, old, n) || regrow(&ilist, old, n) || regrow(&sinks, old, n) || regrow(&wl, old, n) ||
-        regrow(&act, old, n) || regrow(&win, old, n) || regrow(&neg, old, n) || regrow(&ll, 2 * old, 2 * n) ||
-        regrow(&sl, 6 * old, 6 * n) || regrow(&newidx, 0, n) || regrow(&tail, 0, std::max<long>(n, pphys)) ||
-        regrow(&center, old, n) || regrow(&M.fstamp, old, n) || regrow(&M.tstamp, old, n) || regrow(&fq, 0, n) ||
-        regrow(&tl, 0, n) || regrow(&clr, 0, n) || regrow(&M.wbits, 0, n / 32 + 1) ||
-        regrow(&M.wcnt, 0, n / 1024 + 1) || regrow(&M.wsup, 0, n / 32768 + 1) ||
-        regrow(&M.wmeg, 0, n / 1048576 + 1))
+        regrow(&newidx, 0, n) || regrow(&tail, 0, std::max<long>(n, pphys)) || regrow(&center, old, n) ||
+        regrow(&M.fstamp, old, n) || regrow(&fl.q0, 0, n) || regrow(&fl.q1, 0, n) || regrow(&fl.rec, 0, n) ||
+        regrow(&fl.red, 0, 2 * n) || regrow(&fl.wbits, 0, winner_words(n)))
       return GQM_ERR_MEMORY;
-    // winner bitmap and chunk counts are all zero between flip steps
-    cudaMemsetAsync(M.wbits, 0, sizeof(unsigned) * (n / 32 + 1), st);
-    cudaMemsetAsync(M.wcnt, 0, sizeof(int) * (n / 1024 + 1), st);
-    cudaMemsetAsync(M.wsup, 0, sizeof(int) * (n / 32768 + 1), st);
-    cudaMemsetAsync(M.wmeg, 0, sizeof(int) * (n / 1048576 + 1), st);
+    winner_carve(fl, fl.wbits, n);
     if (n > old) {
       cudaMemsetAsync(M.tst + old, 0, n - old, st);
       cudaMemsetAsync(M.tflip + old, 0, n - old, st);
       cudaMemsetAsync(M.tfo + old, 0, n - old, st);
       cudaMemsetAsync(M.tsg + old, 0xff, sizeof(int4) * (n - old), st);
-      cudaMemsetAsync(M.tpos + old, 0xff, sizeof(int) * (n - old), st);
       cudaMemsetAsync(M.fstamp + old, 0, sizeof(int) * (n - old), st);
-      cudaMemsetAsync(M.tstamp + old, 0, sizeof(int) * (n - old), st);
+      cudaMemsetAsync(M.fmark + old, 0xff, sizeof(unsigned long long) * (n - old), st);
+      cudaMemsetAsync(M.emap + old, 0, sizeof(int4) * (n - old), st);
     }
     tphys = n;
     buf_gen++;
@@ -962,7 +942,8 @@ struct Refiner {
     long old = sphys;
     if (n <= old) return GQM_OK;
     if (regrow(&M.s2t, old, n) || regrow(&M.s2seg, old, n) || regrow(&M.enc, old, n) || regrow(&enclist, old, n) ||
-        regrow(&encl2, old, n) || regrow(&smark, old, n) || regrow(&mids, old, n) || regrow(&snap, old, n))
+        regrow(&encl2, old, n) || regrow(&smark, old, n) || regrow(&mids, old, n) || regrow(&snap, old, n) ||
+        regrow(&fl.late, 0, 2 * n))
       return GQM_ERR_MEMORY;
     // new subsegment entries start at epoch 0 so that the first tagged store wins
     cudaMemsetAsync(M.s2t + old, 0, sizeof(s2t_t) * (n - old), st);
@@ -1141,81 +1122,37 @@ struct Refiner {
   DevSlots pslots() const { return DevSlots{emptyp, &ds->pslot}; }
   DevSlots tslots() const { return DevSlots{emptyt, &ds->tslot}; }
 
-  // ---- flip-flop (refine.cu:2328-2490), driven by active sets ----
-  // One step: check (A) -> winners (W) -> link+phase 1 -> phase 2 -> phase 3
-  // -> redundant points -> reset claims -> next A -> loop condition.  Every
-  // count lives in the control block, so the whole loop runs on the device.
-#ifndef GQM_STEP_GRID
-#define GQM_STEP_GRID (148 * 4)
-#endif
-  // steps whose active set has at most this many triangles run in one launch
+  // Launch shape of the flip-flop loop (gqm_tuning).  None of it changes a
+  // result: every step makes the reference's decisions whatever the grid.
 #ifndef GQM_SMALL_STEP
 #define GQM_SMALL_STEP 1024
 #endif
-  // Launch shape of the flip-flop loop (gqm_tuning).  None of it changes a
-  // result: every step makes the reference's decisions whatever the grid.
   struct Tuning {
-    int step_grid = GQM_STEP_GRID;       // blocks of each grid-wide step kernel
-    int small_limit = GQM_SMALL_STEP;    // <= this many active triangles: small-step kernel (0: never)
-    int small_cluster = 1;               // small-step kernel: 1 = one 512-thread block, 8 / 16 = a cluster
-    int check_minb = GQM_WALK_MIN_BLOCKS;  // register budget of the check kernel (blocks per SM)
+    int step_grid = 148 * 4;           // most blocks of a step (beyond one per SM: one per SM)
+    int small_limit = GQM_SMALL_STEP;  // <= this many queued triangles: the small team (0: never)
+    int small_cluster = 1;             // blocks of the small team
+    int check_minb = 2;                // register budget (2: 512 threads per SM, 1: 256)
     bool operator==(const Tuning &o) const {
       return step_grid == o.step_grid && small_limit == o.small_limit && small_cluster == o.small_cluster &&
              check_minb == o.check_minb;
     }
   } tune;
-  template <int PRED>
-  void launch_check(const TouchL &T) {
-    void (*check)(Mesh, const int *, const int *, uint8_t *, TouchL, KTimer *) =
-        tune.check_minb == 1 ? k_check_flip2<PRED, 1> : k_check_flip2<PRED, 2>;
-    KL(check, tune.step_grid, 256)(M, act, &fc->nact, clr, T, ktm);
-  }
-  void flip_body(cudaGraphConditionalHandle h, int graph) {
-    FlipQ Q{fq, &fc->qn, &fc->gen};
-    TouchL T{tl, &fc->tn, &fc->gen};
-    const int g = tune.step_grid;
-    if (pred_mode)
-      launch_check<1>(T);
-    else
-      launch_check<0>(T);
-    KL(k_flip_winner2, g, 256)(M, act, &fc->nact, clr, Q, win, &fc->winn);
-    KL(k_link_phase1, g, 256)(M, win, &fc->winn, ll, sl, &fc->epoch);
-    KL(k_phase2, g, 256)(M, win, &fc->winn, ll, sl);
-    KL(k_phase3q, g, 256)(M, win, &fc->winn, sl, Q);
-    KL(k_mark_red_steiner_q, g, 256)(M, tl, &fc->tn, Q);
-    KL(k_flip_reset_filter, g, 256)(M, tl, &fc->tn, fq, &fc->qn, act, &fc->nact_next);
-    KL(k_flip_cond, 1, 32)(fc, h, graph);
-    // the following small steps in one block (batch.cu) or one cluster
-    // (flipcl.cu), which re-sets the condition
-    if (tune.small_limit <= 0) return;
-    if (tune.small_cluster > 1)
-      gqm_flip_small_cl_launch(&M, sizeof(M), fc, pred_mode, act, clr, win, ll, sl, fq, tl, tune.small_limit,
-                               tune.small_cluster, st, h, graph, stm);
-    else
-      gqm_flip_small_launch(&M, sizeof(M), fc, pred_mode, act, clr, win, ll, sl, fq, tl, tune.small_limit, st, h,
-                            graph, stm);
-  }
-  // kernels one grid step of the loop body launches (with its condition kernel)
-  int step_kernels() const { return tune.small_limit > 0 ? 9 : 8; }
+  int loop_blocks[3] = {0, 0, 0};  // most resident blocks of the loop's launch, by register budget (0: not asked yet)
 
-  // ---- flip-flop (refine.cu:2328-2490) over the triangles flagged below last_triangle ----
+  // ---- flip-flop (refine.cu:2328-2490) over the triangles flagged since the last loop ----
   int flip_flop() {
     NvtxRange nvtx("gqm:flip_flop");
-    DLAUNCH(k_flip_entry_reset, M, DevInt{&ds->last_triangle});
-    compact_dev(PNotNullFlag{M.tst, M.tflip}, Ident{}, &ds->last_triangle, act, &fc->nact);
-    return cond_node(
-        true,
-        [&](cudaGraphConditionalHandle h, int graph) {
-          KL(k_flip_prep, 1, 32)(fc, h, graph);
-          count_launch(1);
-        },
-        [&](cudaGraphConditionalHandle h, int graph) {
-          flip_body(h, graph);
-          // in a graph the steps are counted after the run (FlipCtl::steps)
-          if (!capturing) stats.kernel_launches += step_kernels();
-          return GQM_OK;
-        },
-        &fc->cond, true);
+    count_launch(1);
+    return gqm_flip_loop_launch(&M, sizeof(M), &fl, sizeof(fl), bars, &ds->team, pred_mode,
+                                loop_blocks[tune.check_minb], tune.check_minb, tune.small_limit, tune.small_cluster,
+                                ktm, stm, st);
+  }
+  // Blocks that a refinement's flip loops use: one per 1,024 input triangles,
+  // at most one per SM (or step_grid).  A step's barriers cost more the more
+  // blocks take part, and a small input's steps never fill a large team.
+  int team_blocks(int nt) const {
+    const int most = std::min(tune.step_grid, loop_blocks[tune.check_minb]);
+    return std::max(1, std::min(most, (nt + 1023) / 1024));
   }
 
   // ---- splitEncsegs (refine.cu:3180-3778) ----
@@ -1228,7 +1165,7 @@ struct Refiner {
       DLAUNCH(k_copy, smark, enclist, &ds->nenc);
       compact_dev(PNonNeg{smark}, ValueOf{smark}, &ds->nmark, mids, &ds->ndel);
       int rc = dev_while(CondDelete{}, [&] {
-        DLAUNCH(k_mark_redundant, M, smark, mids, &ds->ndel);
+        DLAUNCH(k_mark_redundant, M, smark, mids, &ds->ndel, fl);
         int r = flip_flop();
         if (r) return r;
         compact_dev(PNonNeg{smark}, ValueOf{smark}, &ds->nmark, mids, &ds->ndel);
@@ -1250,7 +1187,7 @@ struct Refiner {
         KL(k_bump_epoch, 1, 32)(fc);
         count_launch(1);
         DLAUNCH(k_insert_mid, M, mids, &ds->nmid, smark, snap, pslots(), tslots(), DevInt{&ds->last_subseg},
-                &fc->epoch, dctr + 1);
+                fl, dctr + 1);
         if (explore) DLAUNCH(k_explore_mid_post, M, mids, &ds->nmid, pslots(), ex);
         DLAUNCH(k_update_mid_nbrs, M, mids, &ds->nmid, smark, enclist);
         compact_dev(PNonNeg{smark}, Ident{}, &ds->nenc, mids, &ds->nmid);
@@ -1301,7 +1238,7 @@ struct Refiner {
     DLAUNCH(k_reset_steiner, M, wl, &ds->nst, sinks);
     KL(k_bump_epoch, 1, 32)(fc);
     count_launch(1);
-    DLAUNCH(k_insert_steiner, M, wl, &ds->nst, sinks, center, pslots(), tslots(), &fc->epoch, dctr + 0);
+    DLAUNCH(k_insert_steiner, M, wl, &ds->nst, sinks, center, pslots(), tslots(), fl, dctr + 0);
     if (explore) DLAUNCH(k_explore_steiner, M, wl, &ds->nst, center, pslots(), ex);
     DLAUNCH(k_update_steiner_nbrs, M, wl, &ds->nst, sinks);
     DSTEP((ConsumeSlots{&ds->nst, 2}));
@@ -1590,20 +1527,13 @@ struct Refiner {
     if (ns) cudaMemcpyAsync(segs, dseg_in, sizeof(int2) * ns, cudaMemcpyDeviceToDevice, st);
     M.segs = segs;
     cudaMemsetAsync(M.s2t, 0, sizeof(s2t_t) * sphys, st);
-    if (M.wbits) {  // left set only by a run that stopped inside a flip step
-      cudaMemsetAsync(M.wbits, 0, sizeof(unsigned) * (tphys / 32 + 1), st);
-      cudaMemsetAsync(M.wcnt, 0, sizeof(int) * (tphys / 1024 + 1), st);
-      cudaMemsetAsync(M.wsup, 0, sizeof(int) * (tphys / 32768 + 1), st);
-      cudaMemsetAsync(M.wmeg, 0, sizeof(int) * (tphys / 1048576 + 1), st);
-    }
+    cudaMemsetAsync(bars, 0, gqm_flip_bar_bytes(), st);
     cudaMemsetAsync(M.err, 0, sizeof(int), st);
     cudaMemsetAsync(dctr, 0, sizeof(unsigned long long) * 8, st);
     {
       const unsigned long long zero = 0;
       cudaMemcpyToSymbolAsync(g_incircle_fallbacks, &zero, sizeof(zero), 0, cudaMemcpyHostToDevice, st);
-      // the small-step kernels' counters (their own translation units)
-      gqm_fallbacks_cta(nullptr, 1, st);
-      gqm_fallbacks_cluster(nullptr, 1, st);
+      gqm_fallbacks_cluster(nullptr, 1, st);  // the flip loop's counter (its own translation unit)
     }
     KL(k_ctl_reset, 1, 32)(fc, 64 * max_rounds, M.err);
     LAUNCH(k_check_input, std::max(np, nt), (const double2 *)dpts, np, dtri_in, dnbr_in, nt, dseg_in, ns, M.err);
@@ -1656,6 +1586,7 @@ struct Refiner {
     hds.pointblock = pointblock;
     hds.triblock = triblock;
     hds.max_rounds = max_rounds;
+    hds.team = team_blocks(nt);
     cudaMemcpyAsync(ds, &hds, sizeof(DState), cudaMemcpyHostToDevice, st);
     rc = run_refinement();
     if (rc == 0) {
@@ -1704,10 +1635,6 @@ struct Refiner {
     FlipCtl hf;
     cudaMemcpy(&hf, fc, sizeof(hf), cudaMemcpyDeviceToHost);
     stats.flip_steps = hf.steps;
-    // with the graph, the kernels of every grid step of the flip-flop loops (a
-    // grid step, its condition and the single-block kernel that runs the small
-    // steps after it) are added here
-    if (use_graph) stats.kernel_launches += (long long)step_kernels() * (hf.steps - hf.small_steps);
     for (int b = 0; b < kFlipProfileBins; ++b) {
       flip_prof_steps[b] = (long long)hf.prof_steps[b];
       flip_prof_items[b] = (long long)hf.prof_items[b];
@@ -1717,7 +1644,6 @@ struct Refiner {
     {
       unsigned long long fb = 0;
       cudaMemcpyFromSymbol(&fb, g_incircle_fallbacks, sizeof(fb));
-      gqm_fallbacks_cta(&fb, 0, st);
       gqm_fallbacks_cluster(&fb, 0, st);
       stats.exact_fallbacks = (long long)fb;
     }
@@ -1741,7 +1667,7 @@ struct Refiner {
     if (grow_dev(&d_out, &d_out_cap, bytes) || grow_pinned(bytes)) return GQM_ERR_MEMORY;
     cudaMemcpyAsync(d_out, M.pts, 16 * (size_t)np, cudaMemcpyDeviceToDevice, st);
     LAUNCH(k_emit_output, std::max(nt, ns), M, (int)nt, (int)ns, (int *)(d_out + o_tri), (int *)(d_out + o_nbr),
-           (int *)(d_out + o_seg), (uint8_t *)(d_out + o_ts));
+           (int *)(d_out + o_seg), (uint8_t *)(d_out + o_ts), (const FlipCtl *)fc);
     LAUNCH(k_emit_pstatus, np, M, (int)np, (uint8_t *)(d_out + o_ps));
     if (char *blk = pool_take(bytes)) {  // straight into a pinned block the caller owns until gqm_free_result
       cudaMemcpyAsync(blk, d_out, bytes, cudaMemcpyDeviceToHost, st);
@@ -1900,10 +1826,6 @@ int gqm_context_set_tuning(gqm_context *ctx, const gqm_tuning *t) {
   if (t->small_cluster > 1) n.small_cluster = t->small_cluster;
   if (t->check_blocks_per_sm < 0 || t->check_blocks_per_sm > 2) return GQM_ERR_ARGUMENT;
   if (t->check_blocks_per_sm > 0) n.check_minb = t->check_blocks_per_sm;
-  if (n.small_cluster > 1) {
-    if (cudaSetDevice(ctx->r.device) != cudaSuccess) return GQM_ERR_CUDA;
-    if (!gqm_flip_cluster_ok(n.small_cluster)) return GQM_ERR_CUDA;
-  }
   ctx->r.tune = n;
   return GQM_OK;
 }
@@ -2274,7 +2196,7 @@ static int noalloc_staging(int device, unsigned char **p) {
 
 // k_emit_output / k_emit_pstatus writing into the staging array.  Every row
 // that is copied out is written first, so nothing has to start at zero.
-__global__ void k_emit_output_staged(Mesh M, int np, int nt, int ns, unsigned char *stage) {
+__global__ void k_emit_output_staged(Mesh M, int np, int nt, int ns, unsigned char *stage, const FlipCtl *c) {
   int *tri = reinterpret_cast<int *>(stage + kNoAllocTri);
   int *nbr = reinterpret_cast<int *>(stage + kNoAllocNbr);
   int *seg = reinterpret_cast<int *>(stage + kNoAllocSeg);
@@ -2289,7 +2211,7 @@ __global__ void k_emit_output_staged(Mesh M, int np, int nt, int ns, unsigned ch
       nbr[3 * i] = dtri(nb.x);
       nbr[3 * i + 1] = dtri(nb.y);
       nbr[3 * i + 2] = dtri(nb.z);
-      ts[i] = (uint8_t)((M.tst[i] & 7) | (M.tflip[i] ? 8 : 0) | (M.tfo[i] << 4));
+      ts[i] = status_byte(M, i, c->ran);
     }
     if (i < ns) {
       int o = s2t_get(M, i);
@@ -2322,7 +2244,7 @@ extern "C" int gqm_context_result_noalloc(gqm_context *ctx, gqm_cdt_out *out) {
   if (rc) return rc;
   cudaStream_t st = R.st;
   int work = std::max(std::max(nt, ns), np);
-  KL(gqm::k_emit_output_staged, gqm::Refiner::grid_for(work), 256)(R.M, np, nt, ns, stage);
+  KL(gqm::k_emit_output_staged, gqm::Refiner::grid_for(work), 256)(R.M, np, nt, ns, stage, R.fc);
   if (cudaGetLastError() != cudaSuccess) return GQM_ERR_CUDA;
   // errors reported when a copy is issued (an invalid host pointer, for one)
   // are not sticky, so each copy's status is checked here: a failed call

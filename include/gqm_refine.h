@@ -132,22 +132,20 @@ int gqm_context_result(gqm_context *ctx, gqm_cdt_out *out);
 /* Sizes of the last result without copying it. */
 int gqm_context_result_sizes(gqm_context *ctx, int *npoints, int *ntriangles, int *nsegments);
 /* Measurement probe (no counterpart in the reference).  While enabled, the
- * two kernels that take most of the device time, the grid-wide flip-step check
- * kernel and the small-step kernel (whole flip steps of small active sets in
- * one launch), timestamp every launch on the device: from its first block's
- * start to its last block's end (%globaltimer); the flip-flop loops are timed
- * on the device as well, from entry to their last step.  gqm_context_probe(ctx, 1)
- * resets and enables, (ctx, 0) disables; gqm_context_probe_read sums since the
- * reset. */
+ * flip-flop loops are timed on the device (%globaltimer, by the launch's lead
+ * thread): each loop from entry to its last step, the check phase of every step
+ * that all blocks run (to the barrier behind it), and every run of small steps
+ * by the small team.  gqm_context_probe(ctx, 1) resets and enables, (ctx, 0)
+ * disables; gqm_context_probe_read sums since the reset. */
 typedef struct {
-  long long check_launches; /* launches of the flip-step check kernel */
+  long long check_launches; /* check phases (steps run by all blocks) */
   long long check_items;    /* active triangles they checked */
   double check_ms;          /* their summed execution time */
   long long loop_launches;  /* flip-flop loops run */
   double loop_ms;           /* their summed device time (%globaltimer at loop entry and end) */
-  long long first_items[4]; /* active triangles of the first four check launches */
-  long long small_launches; /* launches of the small-step kernel */
-  long long small_items;    /* active triangles of the flip steps they ran */
+  long long first_items[4]; /* active triangles of the first four check phases */
+  long long small_launches; /* runs of small steps */
+  long long small_items;    /* queued triangles of the flip steps they ran */
   long long small_winners;  /* flips and flops those steps applied */
   double small_ms;          /* their summed execution time */
 } gqm_probe;
@@ -168,17 +166,16 @@ void *gqm_context_stream(gqm_context *ctx);
  * result: every flip step makes the reference's decisions whatever the launch
  * shape.  Zero in a field means its default. */
 typedef struct {
-  int step_grid;           /* blocks of 256 threads of each grid-wide flip-step kernel (default 592, 4 per SM) */
-  int small_limit;         /* flip steps of at most this many active triangles run inside one launch of the
-                              small-step kernel (default 1024; negative: never) */
-  int small_cluster;       /* small-step kernel: 1 = one block of 512 threads (default); 8 or 16 = one
-                              thread-block cluster of that many 256-thread blocks */
-  int check_blocks_per_sm; /* register budget of the flip-step check kernel: 2 resident 256-thread blocks
-                              per SM (default; at most 128 registers) or 1 (up to 255) */
+  int step_grid;           /* most blocks of a flip step (default 592; never more than one per SM, nor than
+                              one per 1,024 input triangles) */
+  int small_limit;         /* flip steps of at most this many queued triangles are run by the small team
+                              (default 1024; negative: never) */
+  int small_cluster;       /* blocks of the small team: 1 (default; its lists in shared memory), 8 or 16 */
+  int check_blocks_per_sm; /* register budget of the flip loop: 2 = 512 threads per SM at most 128 registers
+                              each (default), 1 = 256 threads at up to 255 */
 } gqm_tuning;
 /* Set / read a context's launch shape.  Set returns GQM_ERR_ARGUMENT for a
- * value out of range and GQM_ERR_CUDA when the device cannot run the requested
- * cluster size; the context keeps its previous shape then. */
+ * value out of range; the context keeps its previous shape then. */
 int gqm_context_set_tuning(gqm_context *ctx, const gqm_tuning *t);
 int gqm_context_get_tuning(gqm_context *ctx, gqm_tuning *t);
 /* Autotuner (no counterpart in the reference): refines `in` (host or device
