@@ -1,18 +1,14 @@
-// Batched refinement of many independent domains in one persistent launch.
+// Batched refinement of many independent domains in one persistent launch, and
+// the refinement of one domain in one launch.
 //
-// Each thread block is a complete refiner for one domain at a time: the
-// driver of refine.cu (GPU_Refine_Quality's control flow,
-// GPU_Refine/refine.cu:6500-7139, with its free-slot bookkeeping) runs on the
-// device, every thread of the block executing the same scalar control flow,
-// and every pipeline step is the same kernel source as the single-domain path
-// (kernels.cuh compiled in CTA mode: the block's threads stride over the
-// domain's items and __syncthreads() separates the steps).  Blocks take
-// domains from a queue ordered largest first (one atomic counter), so the
-// whole batch, including every domain's round loop and flip-flop loop, is
-// decided on the device: no host round trip and no launch per step.
+// Each team of thread blocks is a complete refiner for one domain at a time
+// (engine.cuh).  Teams take domains from a queue ordered largest first (one
+// atomic counter), so the whole batch, including every domain's round loop and
+// flip-flop loop, is decided on the device: no host round trip and no launch
+// per step.
 //
 // A domain's result is the one the single-domain path returns for it: the
-// same steps run in the same order on the same slot discipline.  Each block
+// same steps run in the same order on the same slot discipline.  Each team
 // owns one scratch arena sized for the largest domain of the batch; a domain
 // whose mesh would outgrow its arena stops with GQM_ERR_ARENA and is refined
 // again by the single-domain path on the host side of the call.
@@ -26,109 +22,18 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <mutex>
+#include <queue>
 #include <thread>
 #include <vector>
 
 #include "host_copy.h"
 
 #include "../../include/gqm_refine.h"
-#include "kernels.cuh"
+#include "engine.cuh"
 
 namespace gqm {
-
-// ---------------------------------------------------------------------------
-// Block-wide helpers (every thread of the block calls them)
-// ---------------------------------------------------------------------------
-
-// Ordered compaction: out[k] = map(i) for the k-th i in [lo, hi) with pred(i),
-// ascending; returns the count (the same value in every thread).  scan holds
-// 33 ints of shared memory.
-template <class F, class Mp>
-__device__ int cta_compact(F f, Mp m, int lo, int hi, int *out, int *scan) {
-  const int lane = (int)(threadIdx.x & 31u), w = (int)(threadIdx.x >> 5);
-  const int nw = (int)((blockDim.x + 31u) >> 5);
-  int base = 0;
-  for (int t0 = lo; t0 < hi; t0 += (int)blockDim.x) {
-    const int i = t0 + (int)threadIdx.x;
-    const bool p = i < hi && f(i);
-    const unsigned b = __ballot_sync(0xffffffffu, p);
-    if (lane == 0) scan[w] = __popc(b);
-    __syncthreads();
-    if (w == 0) {
-      const int v = lane < nw ? scan[lane] : 0;
-      int x = v;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-      }
-      scan[lane] = x - v;
-      const int total = __shfl_sync(0xffffffffu, x, 31);
-      if (lane == 0) scan[32] = total;
-    }
-    __syncthreads();
-    if (p) out[base + scan[w] + __popc(b & ((1u << lane) - 1u))] = m(i);
-    base += scan[32];
-    __syncthreads();
-  }
-  return base;
-}
-template <class T>
-__device__ __forceinline__ void cta_fill(T *a, long n, T v) {
-  for (long i = threadIdx.x; i < n; i += blockDim.x) a[i] = v;
-}
-__device__ __forceinline__ void cta_copy(int *dst, const int *src, int n) {
-  for (int i = (int)threadIdx.x; i < n; i += (int)blockDim.x) dst[i] = src[i];
-}
-#define SYNC() __syncthreads()
-
-// predicates and maps of the compactions (the same as refine.cu's)
-struct Ident {
-  __device__ int operator()(int i) const { return i; }
-};
-struct ValueOf {
-  const int *a;
-  __device__ int operator()(int i) const { return a[i]; }
-};
-struct PNotNullFlag {
-  const uint8_t *tst, *flag;
-  __device__ bool operator()(int i) const { return (tst[i] & TS_NOTNULL) && flag[i]; }
-};
-struct PNonNeg {
-  const int *a;
-  __device__ bool operator()(int i) const { return a[i] >= 0; }
-};
-struct PBad {
-  const uint8_t *tst;
-  __device__ bool operator()(int i) const { return (tst[i] & (TS_NOTNULL | TS_BAD)) == (TS_NOTNULL | TS_BAD); }
-};
-struct PTriNull {
-  const uint8_t *tst;
-  __device__ bool operator()(int i) const { return !(tst[i] & TS_NOTNULL); }
-};
-struct PTriLive {
-  const uint8_t *tst;
-  __device__ bool operator()(int i) const { return (tst[i] & TS_NOTNULL) != 0; }
-};
-struct PPtDeleted {
-  const uint8_t *ps;
-  __device__ bool operator()(int i) const { return (ps[i] & PS_DELETED) != 0; }
-};
-struct PPtLive {
-  const uint8_t *ps;
-  __device__ bool operator()(int i) const { return !(ps[i] & PS_DELETED); }
-};
-
-// The block as a team of flip_step.
-struct BlockTeam {
-  __device__ __forceinline__ int tid() const { return (int)threadIdx.x; }
-  __device__ __forceinline__ int size() const { return (int)blockDim.x; }
-  __device__ __forceinline__ bool lead() const { return threadIdx.x == 0; }
-  __device__ __forceinline__ bool sync() {
-    __syncthreads();
-    return true;
-  }
-};
 
 // ---------------------------------------------------------------------------
 // One domain of a batch, in device memory.  The host fills the inputs, the
@@ -156,14 +61,9 @@ struct Job {
   double goodcos2;
 };
 
-// Capacities of one domain: the logical capacity starts as in the
-// single-domain path (refine.cu:6543-6544: pointblock = (int)(0.5 N),
-// triblock = 2 pointblock); the physical sizes leave room for four more point
-// blocks and five more triangle blocks of growth, and for eight subsegments
-// per input segment plus one per two input points.
-struct Caps {
-  long pointblock, triblock, pphys, tphys, sphys, cav_cap, hsz;
-};
+// Arena sizes of one domain: room for four more point blocks and five more
+// triangle blocks of growth, and for eight subsegments per input segment plus
+// one per two input points.
 __host__ __device__ inline Caps caps_of(int np, int nt, int ns) {
   Caps c;
   c.pointblock = (int)(np * 0.5);
@@ -184,16 +84,6 @@ __host__ __device__ inline Caps caps_of(int np, int nt, int ns) {
   return c;
 }
 
-// Scratch of one domain, carved from its block's arena.
-struct Scratch {
-  Mesh M;
-  int *emptyt, *bad, *imark, *ilist, *sinks, *wl, *newidx, *tail;
-  int *emptyp, *pnew, *enclist, *encl2, *smark, *mids, *snap, *cav, *cavn;
-  FlipLists fl;
-  double2 *center;
-  unsigned long long *hkeys;
-  int *hvals, *s2ti;
-};
 // Walks the arena layout: with base == 0 it only measures (host), otherwise it
 // assigns every pointer of S (device).  Every array starts on 256 bytes.
 struct Cursor {
@@ -278,417 +168,154 @@ inline size_t arena_bytes(const Caps &c) {
   return (a.off + 255) & ~(size_t)255;
 }
 
-// ---------------------------------------------------------------------------
-// The device-side driver: Refiner (refine.cu) restated for one thread block.
-// Every thread runs the same control flow on the same scalars; counts come
-// from block-wide compactions or from the shared control block, read after a
-// barrier.  Device pointers to counts (the kernels' `dn`) point into shared
-// memory.
-// ---------------------------------------------------------------------------
-enum { C_LIST0 = 0, C_LIST1, C_LIST2, C_MISC };
-
-struct Shared {
-  Scratch S;
-  FlipCtl fc;
-  unsigned long long ctr[6];  // Steiner points, midpoints, -, -, learned candidates, learned points
-  double gc[2];
-  int cnt[8];
-  int scan[33];
-  int err;
-  int job;
-};
-
+// One domain of a batch: the refinement, then its output block.
 template <int PRED>
-struct Cta {
-  Shared &sh;
-  Caps c;
-  long pcap, tcap;
-  int last_point, last_triangle, last_subseg;
-  int nempty_p, nempty_t, lenp, lent;
-  int offcenter, offconstant, placement;
-  MlpDev mlp;
-  long long max_rounds;
+__device__ int run_job(Engine<PRED> &R, Job &J) {
+  BlockState &sh = R.sh;
+  TeamState &ts = R.ts;
+  GridTeam &T = R.T;
+  Scratch &S = sh.S;
+  R.c = caps_of(J.np, J.nt, J.ns);
+  if (threadIdx.x == 0) {
+    S.M.segs = J.seg;
+    S.M.err = &ts.err;
+    S.fl.c = &ts.fc;
+  }
+  if (R.lead()) {
+    ts.err = 0;
+    for (int i = 0; i < 6; ++i) ts.ctr[i] = 0;
+    ts.fc.gen = 0;
+    ts.fc.epoch = 0;
+    ctl_reset(&ts.fc, 64 * J.max_rounds, &ts.err, true);
+  }
+  // stamps and claims start afresh for every domain
+  __syncthreads();
+  R.fill(S.M.fstamp, R.c.tphys, 0);
+  R.fill(S.M.fmark, R.c.tphys, ~0ull);
+  R.fill(S.M.emap, R.c.tphys, make_int4(0, 0, 0, 0));
+  TSYNC();
+  double gc = 0.0;
+  int rc = R.refine(J, J.theta, &gc);
+  if (R.lead()) J.goodcos2 = gc;
+  int out_np = 0, out_nt = 0;
+  if (rc == GQM_OK) rc = R.compact_output(&out_np, &out_nt);
+  if (rc == GQM_ERR_TOPOLOGY) return rc;
+  if (const int e = R.read_err()) rc = rc ? rc : e;
+  if (rc == GQM_OK) {
+    const OutLayout L = out_layout(out_np, out_nt, R.last_subseg);
+    if (R.lead()) {
+      const unsigned long long off = atomicAdd(J.oused, (unsigned long long)L.bytes);
+      ts.part[0][0] = off + L.bytes <= J.ocap ? 0 : GQM_ERR_ARENA;
+      J.ooff = off;
+    }
+    TSYNC();
+    rc = vload(&ts.part[0][0]);
+    if (rc == GQM_OK) {
+      char *o = J.obase + *(volatile unsigned long long *)&J.ooff;
+      k_emit_output(S.M, out_nt, R.last_subseg, reinterpret_cast<int *>(o + L.tri), reinterpret_cast<int *>(o + L.nbr),
+                    reinterpret_cast<int *>(o + L.seg), reinterpret_cast<uint8_t *>(o + L.ts), &ts.fc);
+      k_emit_pstatus(S.M, out_np, reinterpret_cast<uint8_t *>(o + L.ps));
+      double2 *op = reinterpret_cast<double2 *>(o + L.pts);
+      for (int i = T.tid(); i < out_np; i += T.size()) op[i] = S.M.pts[i];
+    }
+    TSYNC();
+  }
+  if (R.lead()) {
+    J.out_np = out_np;
+    J.out_nt = out_nt;
+    J.out_ns = R.last_subseg;
+    J.rounds = R.rounds;
+    J.bad_total = R.bad_total;
+    J.flip_steps = ts.fc.steps;
+    J.steiner = (long long)ts.ctr[0];
+    J.midpoints = (long long)ts.ctr[1];
+    J.exact_fallbacks = (long long)ts.ctr[2];
+    J.learned_candidates = (long long)ts.ctr[4];
+    J.learned_used = (long long)ts.ctr[5];
+  }
+  return rc;
+}
 
-  __device__ bool lead() const { return threadIdx.x == 0; }
-  template <class F, class Mp>
-  __device__ int compact(F f, Mp m, int lo, int hi, int *out) {
-    return cta_compact(f, m, lo, hi, out, sh.scan);
-  }
-  // the device error word, read by every thread before anyone can change it
-  // again (the barrier keeps the block's decision on it uniform)
-  __device__ int read_err() {
-    const int e = sh.err;
-    SYNC();
-    return e;
-  }
-  // a count that the next step reads through a pointer
-  __device__ int *publish(int slot, int v) {
-    if (lead()) sh.cnt[slot] = v;
-    SYNC();
-    return sh.cnt + slot;
-  }
-
-  // updateEmptyPoints / updateEmptyTriangles (refine.cu:149-197)
-  __device__ int refresh_points() {
-    lenp = compact(PPtDeleted{sh.S.M.ps}, Ident{}, 0, (int)pcap, sh.S.emptyp);
-    return lenp;
-  }
-  __device__ int refresh_tris() {
-    lent = compact(PTriNull{sh.S.M.tst}, Ident{}, 0, (int)tcap, sh.S.emptyt);
-    return lent;
-  }
-  // growth steps of refine.cu:3408-3444 / 5259-5296 on the logical capacity
-  __device__ int ensure_slots(int npts, int ntris) {
-    if (npts > nempty_p) {
-      nempty_p = refresh_points();
-      long num = 0;
-      while (npts > nempty_p + num * c.pointblock) num++;
-      if (num) {
-        long ncap = pcap + num * c.pointblock;
-        if (ncap > c.pphys) return GQM_ERR_ARENA;
-        pcap = ncap;
-        nempty_p = refresh_points();
-      }
-    }
-    if (ntris > nempty_t) {
-      nempty_t = refresh_tris();
-      long num = 0;
-      while (ntris > nempty_t + num * c.triblock) num++;
-      if (num) {
-        long ncap = tcap + num * c.triblock;
-        if (ncap > c.tphys) return GQM_ERR_ARENA;
-        tcap = ncap;
-        nempty_t = refresh_tris();
-      }
-    }
-    return GQM_OK;
-  }
-  // slot bookkeeping after an insertion batch (refine.cu:3545-3559, 5354-5368)
-  __device__ void consume_slots(int npts, int ntris) {
-    int slot_after = (int)(pcap - last_point);
-    int slot_before = nempty_p - slot_after;
-    if (slot_before < npts) last_point += npts - slot_before;
-    nempty_p -= npts;
-    slot_after = (int)(tcap - last_triangle);
-    slot_before = nempty_t - slot_after;
-    if (slot_before < ntris) last_triangle += ntris - slot_before;
-    nempty_t -= ntris;
-  }
-  __device__ const int *pslots() const { return sh.S.emptyp + (lenp - nempty_p); }
-  __device__ const int *tslots() const { return sh.S.emptyt + (lent - nempty_t); }
-
-  // ---- flip-flop (refine.cu:2328-2490) ----
-  __device__ __noinline__ int flip_flop() {
-    const FlipLists &L = sh.S.fl;
-    FlipCtl *fc = &sh.fc;
-    BlockTeam T;
-    FlipRegs R{fc->gen, fc->epoch, fc->steps};
-    const int entry = R.steps;
-    for (;;) {
-      const int n = vload(&fc->cnt.qn[R.gen & 1]);
-      if (n == 0) break;
-      if (flip_step<PRED>(sh.S.M, L, &fc->cnt, R, entry, T, (R.gen & 1) ? L.q1 : L.q0, n, L.rec, nullptr, nullptr) !=
-          FLIP_GO)
-        break;
-    }
-    SYNC();
-    if (lead()) {
-      flip_close(fc, R);
-      fc->ran++;
-    }
-    SYNC();
-    return GQM_OK;  // errors raised on the device are read by the round loop
-  }
-
-  // ---- splitEncsegs (refine.cu:3180-3778) ----
-  __device__ int split_encsegs() {
-    Scratch &S = sh.S;
-    long long outer = 0;
-    for (;;) {
-      int nenc = compact(PNonNeg{S.M.enc}, Ident{}, 0, last_subseg, S.enclist);
-      if (nenc == 0) break;
-      if (++outer > max_rounds) return GQM_ERR_ROUND_LIMIT;
-      // delete free Steiner points inside diametral circles
-      cta_copy(S.smark, S.enclist, nenc);
-      SYNC();
-      int nmark = nenc;
-      long long inner = 0;
-      for (;;) {
-        int ndel = compact(PNonNeg{S.smark}, ValueOf{S.smark}, 0, nmark, S.mids);
-        if (ndel == 0) break;
-        if (++inner > max_rounds) return GQM_ERR_ROUND_LIMIT;
-        nmark = ndel;
-        k_mark_redundant(S.M, S.smark, S.mids, publish(C_LIST1, ndel), S.fl);
-        SYNC();
-        int rc = flip_flop();
-        if (rc) return rc;
-      }
-      int rc = ensure_slots(nenc, 2 * nenc);
-      if (rc) return rc;
-      if (last_subseg + nenc > c.sphys) return GQM_ERR_ARENA;
-      cta_fill(S.M.enc + last_subseg, nenc, -1);
-      cta_copy(S.smark, S.enclist, nenc);
-      SYNC();
-      long long mid_iter = 0;
-      for (;;) {
-        int nmid = compact(PNonNeg{S.smark}, Ident{}, 0, nenc, S.mids);
-        if (nmid == 0) break;
-        if (++mid_iter > 64 * max_rounds) return GQM_ERR_ROUND_LIMIT;
-        int *dn = publish(C_LIST1, nmid);
-        k_reset_mid(S.M, S.mids, dn, S.smark);
-        SYNC();
-        k_mark_mid(S.M, S.mids, dn, S.smark);
-        SYNC();
-        k_mid_snapshot(S.M, S.mids, dn, S.smark, S.snap);
-        if (lead()) sh.fc.epoch++;
-        SYNC();
-        k_insert_mid(S.M, S.mids, dn, S.smark, S.snap, pslots(), tslots(), last_subseg, S.fl, sh.ctr + 1);
-        SYNC();
-        k_update_mid_nbrs(S.M, S.mids, dn, S.smark, S.enclist);
-        SYNC();
-      }
-      consume_slots(nenc, 2 * nenc);
-      last_subseg += nenc;
-      rc = flip_flop();
-      if (rc) return rc;
-    }
-    return GQM_OK;
-  }
-
-  // ---- splitTriangles (refine.cu:5107-5547) ----
-  __device__ int split_triangles(int nbad) {
-    Scratch &S = sh.S;
-    int *dn = sh.cnt + C_LIST2;  // number of bad triangles, published by the caller
-    cta_copy(S.imark, S.bad, nbad);
-    cta_copy(S.ilist, S.bad, nbad);
-    k_circumcenter(S.M, S.bad, dn, (double)offconstant, offcenter, S.center);
-    cta_fill(S.M.tmark, last_triangle, kMaxInt);
-    SYNC();
-    if (placement == GQM_PLACE_LEARNED) {
-      k_learned_place(S.M, S.bad, dn, mlp, S.center, sh.ctr + 4);
-      SYNC();
-    }
-    k_locate<PRED>(S.M, S.bad, dn, S.center, S.sinks);
-    SYNC();
-    k_remove_losers(S.M, S.bad, dn, S.sinks, S.imark);
-    SYNC();
-    cta_fill(S.M.tmark, last_triangle, kMaxInt);
-    SYNC();
-    if (nbad > c.cav_cap) return GQM_ERR_ARENA;
-    k_cavity_mark<PRED>(S.M, dn, S.sinks, S.center, S.imark, S.ilist, S.cav, S.cavn, nbad);
-    SYNC();
-    k_cavity_check(S.M, dn, S.cav, S.cavn, nbad, S.imark, S.ilist);
-    SYNC();
-    int nst = compact(PNonNeg{S.imark}, Ident{}, 0, nbad, S.wl);
-    int *dw = publish(C_LIST1, nst);
-    cta_fill(S.encl2, last_subseg, -1);
-    SYNC();
-    k_mark_onsegs(S.M, S.wl, dw, S.sinks, S.encl2);
-    SYNC();
-    int rc = ensure_slots(nst, 2 * nst);
-    if (rc) return rc;
-    k_reset_steiner(S.M, S.wl, dw, S.sinks);
-    if (lead()) sh.fc.epoch++;
-    SYNC();
-    k_insert_steiner(S.M, S.wl, dw, S.sinks, S.center, pslots(), tslots(), S.fl, sh.ctr + 0);
-    SYNC();
-    k_update_steiner_nbrs(S.M, S.wl, dw, S.sinks);
-    SYNC();
-    consume_slots(nst, 2 * nst);
-    rc = flip_flop();
-    if (rc) return rc;
-    k_onsegs_to_enc(S.M, S.encl2, last_subseg);
-    SYNC();
-    return GQM_OK;
-  }
-
-  // ---- output compaction (refine.cu:5758-6428) ----
-  __device__ void compact_output(int &out_np, int &out_nt) {
-    Scratch &S = sh.S;
-    int newn = compact(PTriLive{S.M.tst}, Ident{}, 0, last_triangle, S.tail);
-    k_newidx_init(S.M, S.newidx, last_triangle, newn, S.M.tst, (uint8_t)TS_NOTNULL, false);
-    SYNC();
-    if (newn < last_triangle) {
-      compact(PTriNull{S.M.tst}, Ident{}, 0, newn, S.emptyt);
-      int nmove = compact(PTriLive{S.M.tst}, Ident{}, newn, last_triangle, S.tail);
-      k_compact_tris_move(S.M, S.tail, S.emptyt, publish(C_LIST1, nmove), S.newidx);
-      SYNC();
-      k_fix_nbrs(S.M, S.newidx, newn);
-      k_fix_s2t(S.M, S.newidx, last_subseg);
-      SYNC();
-    }
-    int ntri = newn;
-    int newp = compact(PPtLive{S.M.ps}, Ident{}, 0, last_point, S.pnew);
-    k_newidx_init(S.M, S.pnew, last_point, newp, S.M.ps, (uint8_t)PS_DELETED, true);
-    SYNC();
-    if (newp < last_point) {
-      compact(PPtDeleted{S.M.ps}, Ident{}, 0, newp, S.emptyp);
-      int nmove = compact(PPtLive{S.M.ps}, Ident{}, newp, last_point, S.tail);
-      k_compact_pts_move(S.M, S.tail, S.emptyp, publish(C_LIST1, nmove), S.pnew);
-      SYNC();
-      k_fix_tri_vertices(S.M, S.pnew, ntri);
-      SYNC();
-    }
-    out_np = newp;
-    out_nt = ntri;
-  }
-
-  // ---- the whole refinement of one domain (Refiner::run) ----
-  __device__ int run(Job &J) {
-    Scratch &S = sh.S;
-    const int np = J.np, nt = J.nt, ns = J.ns;
-    c = caps_of(np, nt, ns);
-    offcenter = J.offcenter;
-    offconstant = J.offconstant;
-    placement = J.placement;
-    mlp = J.mlp;
-    max_rounds = J.max_rounds;
-    pcap = np + c.pointblock;
-    tcap = nt + c.triblock;
-    if (lead()) {
-      S.M.segs = J.seg;
-      S.M.err = &sh.err;
-      sh.err = 0;
-      for (int i = 0; i < 6; ++i) sh.ctr[i] = 0;
-      sh.fc.gen = 0;
-      sh.fc.epoch = 0;
-      ctl_reset(&sh.fc, 64 * max_rounds, &sh.err, true);
-      S.fl.c = &sh.fc;
-    }
-    SYNC();
-    // stamps, claims and tags start afresh for every domain
-    cta_fill(S.M.s2t, c.sphys, (s2t_t)0);
-    cta_fill(S.M.fstamp, c.tphys, 0);
-    cta_fill(S.M.fmark, c.tphys, ~0ull);
-    cta_fill(S.M.emap, c.tphys, make_int4(0, 0, 0, 0));
-    k_check_input(J.pts, np, J.tri, J.nbr, nt, reinterpret_cast<const int *>(J.seg), ns, &sh.err);
-    k_goodcos(J.theta, sh.gc);
-    SYNC();
-    if (const int e = read_err()) return e;
-    if (lead()) {
-      S.M.gc2 = sh.gc[0];
-      S.M.mode = J.mode;
-      S.M.max_area = J.max_area;
-      J.goodcos2 = sh.gc[0];
-    }
-    SYNC();
-    k_init_points(S.M, J.pts, np, (int)c.pphys);
-    k_init_tris(S.M, J.tri, J.nbr, nt, (int)c.tphys);
-    cta_fill(S.hkeys, c.hsz, ~0ull);
-    cta_fill(S.s2ti, (long)ns + 1, -1);
-    SYNC();
-    // initSubsegs via a hash of segment endpoints
-    k_seg_hash_insert(J.seg, ns, S.hkeys, S.hvals, (unsigned)(c.hsz - 1));
-    SYNC();
-    k_init_subsegs(S.M, nt, S.hkeys, S.hvals, (unsigned)(c.hsz - 1), S.s2ti);
-    SYNC();
-    k_pack_s2t(S.M, S.s2ti, ns);
-    SYNC();
-    last_point = np;
-    last_triangle = nt;
-    last_subseg = ns;
-    nempty_p = refresh_points();
-    nempty_t = refresh_tris();
-    k_mark_all_encsegs(S.M, ns);
-    SYNC();
-    int rc = split_encsegs();
-    int rounds = 0;
-    long long bad_total = 0;
-    while (rc == 0) {
-      k_mark_bad(S.M, last_triangle);
-      SYNC();
-      int nbad = compact(PBad{S.M.tst}, Ident{}, 0, last_triangle, S.bad);
-      publish(C_LIST2, nbad);
-      if (const int e = read_err()) {
-        rc = e;
-        break;
-      }
-      if (nbad == 0) break;
-      if (rounds >= max_rounds) {
-        rc = GQM_ERR_ROUND_LIMIT;
-        break;
-      }
-      bad_total += nbad;
-      rc = split_triangles(nbad);
-      if (rc) break;
-      rc = split_encsegs();
-      if (rc) break;
-      k_points_old(S.M, last_point);
-      SYNC();
-      rounds++;
-    }
-    if (const int e = read_err()) rc = rc ? rc : e;
-    int out_np = 0, out_nt = 0;
-    if (rc == 0) compact_output(out_np, out_nt);
-    if (const int e = read_err()) rc = rc ? rc : e;
-    if (rc == 0) {
-      const OutLayout L = out_layout(out_np, out_nt, last_subseg);
-      if (lead()) {
-        const unsigned long long off = atomicAdd(J.oused, (unsigned long long)L.bytes);
-        sh.cnt[C_MISC] = off + L.bytes <= J.ocap ? 0 : GQM_ERR_ARENA;
-        J.ooff = off;
-      }
-      SYNC();
-      rc = sh.cnt[C_MISC];
-      if (rc == 0) {
-        char *o = J.obase + J.ooff;
-        k_emit_output(S.M, out_nt, last_subseg, reinterpret_cast<int *>(o + L.tri), reinterpret_cast<int *>(o + L.nbr),
-                      reinterpret_cast<int *>(o + L.seg), reinterpret_cast<uint8_t *>(o + L.ts), &sh.fc);
-        k_emit_pstatus(S.M, out_np, reinterpret_cast<uint8_t *>(o + L.ps));
-        double2 *op = reinterpret_cast<double2 *>(o + L.pts);
-        for (int i = (int)threadIdx.x; i < out_np; i += (int)blockDim.x) op[i] = S.M.pts[i];
-      }
-      SYNC();
-    }
-    if (lead()) {
-      J.out_np = out_np;
-      J.out_nt = out_nt;
-      J.out_ns = last_subseg;
-      J.rounds = rounds;
-      J.bad_total = bad_total;
-      J.flip_steps = sh.fc.steps;
-      J.steiner = (long long)sh.ctr[0];
-      J.midpoints = (long long)sh.ctr[1];
-      J.exact_fallbacks = (long long)sh.ctr[2];
-      J.learned_candidates = (long long)sh.ctr[4];
-      J.learned_used = (long long)sh.ctr[5];
-    }
-    return rc;
-  }
-};
-
-// The persistent batch kernel: each block takes the next domain (largest
-// first) until the queue is empty, refining it in its own arena.
+// The persistent batch kernel: teams of nb consecutive blocks, each taking the
+// next domain (largest first) until the queue is empty, refining it in its own
+// arena.  A team of one block keeps its state in shared memory.
 template <int PRED>
-__device__ void batch_body(Job *jobs, const int *order, int njobs, int *next, char *arenas, size_t arena_stride,
-                           Shared &sh) {
-  char *arena = arenas + (size_t)blockIdx.x * arena_stride;
+__device__ __forceinline__ void batch_body(Job *jobs, const int *order, int njobs, int *next, char *arenas,
+                                           size_t arena_stride, TeamState *teams, int nb, BlockState &sh,
+                                           TeamState &own) {
+  const int team = (int)blockIdx.x / nb;
+  TeamState &ts = nb == 1 ? own : teams[team];
+  if (threadIdx.x == 0) {
+    gqm_team_rank = (int)blockIdx.x % nb;
+    gqm_team_blocks = nb;
+  }
+  __syncthreads();
+  char *arena = arenas + (size_t)team * arena_stride;
+  Engine<PRED> R{sh, ts, GridTeam{&ts.bar, nb, gqm_team_rank, 0ull, &ts.err}, nullptr, nullptr,
+                 kTeamSmallLimit};
   for (;;) {
-    if (threadIdx.x == 0) sh.job = atomicAdd(next, 1);
-    SYNC();
-    const int k = sh.job;
-    SYNC();
+    if (R.lead()) ts.job = atomicAdd(next, 1);
+    if (!R.T.sync()) return;
+    const int k = vload(&ts.job);
+    if (!R.T.sync()) return;
     if (k >= njobs) break;
     Job &J = jobs[order[k]];
     if (threadIdx.x == 0) {
       Cursor a{arena, 0};
       carve(a, sh.S, caps_of(J.np, J.nt, J.ns));
     }
-    SYNC();
-    Cta<PRED> R{sh};
-    const int rc = R.run(J);
-    SYNC();
-    if (threadIdx.x == 0) J.status = rc;
+    __syncthreads();
+    const int rc = run_job(R, J);
+    if (R.lead()) J.status = rc;
+    if (!R.T.sync()) return;
   }
 }
 template <int NT, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_batch(Job *jobs, const int *order, int njobs, int *next, char *arenas,
-                                                    size_t arena_stride, int pred) {
-  __shared__ Shared sh;
+__global__ void __launch_bounds__(NT, MINB)
+    k_batch(Job *jobs, const int *order, int njobs, int *next, char *arenas, size_t arena_stride, TeamState *teams,
+            int nb, int pred) {
+  __shared__ BlockState sh;
+  __shared__ TeamState own;
   if (pred)
-    batch_body<1>(jobs, order, njobs, next, arenas, arena_stride, sh);
+    batch_body<1>(jobs, order, njobs, next, arenas, arena_stride, teams, nb, sh, own);
   else
-    batch_body<0>(jobs, order, njobs, next, arenas, arena_stride, sh);
+    batch_body<0>(jobs, order, njobs, next, arenas, arena_stride, teams, nb, sh, own);
+}
+
+// One domain in the single-domain engine's buffers, by the whole grid.
+template <int PRED>
+__global__ void __launch_bounds__(512, 1)
+    k_refine_one(Scratch S, Caps c, EngineRun *run, TeamState *ts, int small_limit, KTimer *ktm, KTimer *stm) {
+  __shared__ BlockState sh;
+  const int nb = (int)gridDim.x;
+  if (threadIdx.x == 0) {
+    gqm_team_rank = (int)blockIdx.x;
+    gqm_team_blocks = nb;
+    sh.S = S;
+    sh.S.M.segs = run->seg;
+    sh.S.M.err = &ts->err;
+  }
+  __syncthreads();
+  Engine<PRED> R{sh, *ts, GridTeam{&ts->bar, nb, (int)blockIdx.x, 0ull, &ts->err}, ktm, stm, small_limit, c};
+  double gc = 0.0;
+  int out_np = 0, out_nt = 0;
+  int rc = R.refine(*run, run->theta, &gc);
+  if (rc == GQM_OK) rc = R.compact_output(&out_np, &out_nt);
+  if (rc != GQM_ERR_TOPOLOGY)
+    if (const int e = R.read_err()) rc = rc ? rc : e;
+  if (R.lead()) {
+    run->status = rc;
+    run->need_grow = R.need_grow;
+    run->out_np = out_np;
+    run->out_nt = out_nt;
+    run->out_ns = R.last_subseg;
+    run->rounds = R.rounds;
+    run->bad_total = R.bad_total;
+    run->last_point = R.last_point;
+    run->last_triangle = R.last_triangle;
+    run->goodcos2 = gc;
+    for (int i = 0; i < 6; ++i) run->ctr[i] = ts->ctr[i];
+  }
 }
 
 }  // namespace gqm
@@ -699,7 +326,7 @@ __global__ void __launch_bounds__(NT, MINB) k_batch(Job *jobs, const int *order,
 namespace gqm {
 namespace {
 
-typedef void (*BatchFn)(Job *, const int *, int, int *, char *, size_t, int);
+typedef void (*BatchFn)(Job *, const int *, int, int *, char *, size_t, TeamState *, int, int);
 struct Variant {
   int threads, minb;
   BatchFn fn;
@@ -708,7 +335,11 @@ struct Variant {
 const Variant kVariants[] = {{128, 4, k_batch<128, 4>}, {256, 1, k_batch<256, 1>}, {256, 2, k_batch<256, 2>},
                              {512, 1, k_batch<512, 1>}};
 constexpr int kNumVariants = (int)(sizeof(kVariants) / sizeof(kVariants[0]));
-constexpr int kDefaultVariant = 2;
+// one 512-thread block per SM: the fastest on every batch measured (256
+// domains 101 ms against 152, 181 and 355 ms for 256x1, 256x2 and 128x4, 700
+// domains 117 ms against 171, 204 and 393 ms), and the one that forms teams
+constexpr int kTeamVariant = 3;
+constexpr int kDefaultVariant = kTeamVariant;
 
 // Buffers kept per device between calls (grow only).
 struct DevCache {
@@ -717,7 +348,8 @@ struct DevCache {
   cudaStream_t st = nullptr;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   char *d_in = nullptr, *d_out = nullptr, *d_arena = nullptr, *h_in = nullptr, *h_out = nullptr;
-  size_t in_cap = 0, out_cap = 0, arena_cap = 0, h_in_cap = 0, h_out_cap = 0;
+  char *d_teams = nullptr;
+  size_t in_cap = 0, out_cap = 0, arena_cap = 0, h_in_cap = 0, h_out_cap = 0, teams_cap = 0;
   Job *d_jobs = nullptr;
   int *d_order = nullptr;
   int jobs_cap = 0;
@@ -790,6 +422,47 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
   return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
 
+// Blocks per team for a batch on `resident` blocks.  A team of one block keeps
+// every block busy in a large batch, but a block works on its last, or largest,
+// domain alone.  A domain of n points takes a team of nb blocks about
+// L + P / nb: L = 1.35 log2(n) - 8.8 ms for the chain of its steps (at least
+// 1 ms), whatever the team, and P = 0.75 ms per 1,000 points for the work in
+// them (measured: 49,497 points take 48.6, 32.7, 22.1, 16.8, 14.3 and 13.1 ms
+// with 1, 2, 4, 8, 16 and 32 blocks).  The team size is the one whose queue,
+// largest domain first, ends soonest by that.  Measured for domains of 200 to
+// 50,000 points, one block per team and this rule: 16 domains 53.5 and 16.7 ms,
+// 64 domains 79.8 and 33.5 ms, 256 domains 100.2 and 65.6 ms; 700 domains
+// 115.8 ms with one block and 144.3 ms with two.
+constexpr int kTeamSizes[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48};
+int blocks_per_team(const gqm_cdt_in *in, const std::vector<int> &ids, long resident) {
+  std::vector<double> n;
+  for (int d : ids) n.push_back((double)in[d].numberofpoints);
+  std::sort(n.begin(), n.end(), std::greater<double>());
+  int nb = 1;
+  double best = 0.0;
+  for (int k : kTeamSizes) {
+    const size_t teams = std::min((size_t)(resident / k), n.size());
+    if (teams < 1) break;
+    std::priority_queue<double, std::vector<double>, std::greater<double>> ends;
+    double last = 0.0;
+    for (double x : n) {
+      double at = 0.0;
+      if (ends.size() == teams) {
+        at = ends.top();
+        ends.pop();
+      }
+      at += std::max(1.0, 1.35 * std::log2(x) - 8.8) + 0.75e-3 * x / k;
+      ends.push(at);
+      last = std::max(last, at);
+    }
+    if (k == 1 || last < best) {
+      best = last;
+      nb = k;
+    }
+  }
+  return nb;
+}
+
 // One persistent batch over the domains `ids` (all with the same predicate
 // mode) with kernel variant `var`.  Results of domains that finished land in
 // out/stats; the status of each domain in status[d].
@@ -814,7 +487,7 @@ int run_batch(DevCache &C, const std::vector<int> &ids, const gqm_cdt_in *in, gq
   }
   // grid: resident blocks of the variant, bounded by the domains and memory
   const Variant &V = kVariants[var];
-  int per_sm = V.minb;
+  int per_sm = V.minb, nb = 1;
 #ifndef GQM_HOST_EMU
   int occ = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, V.fn, V.threads, 0) == cudaSuccess && occ > 0)
@@ -822,7 +495,9 @@ int run_batch(DevCache &C, const std::vector<int> &ids, const gqm_cdt_in *in, gq
   else
     cudaGetLastError();
 #endif
-  long grid = std::min<long>((long)C.sms * per_sm, n);
+  const long resident = (long)C.sms * per_sm;
+  if (var == kTeamVariant) nb = blocks_per_team(in, ids, resident);
+  long grid = std::min<long>(resident / nb, n);  // teams
 #ifndef GQM_HOST_EMU
   size_t freeb = 0, totb = 0;
   cudaMemGetInfo(&freeb, &totb);
@@ -837,6 +512,9 @@ int run_batch(DevCache &C, const std::vector<int> &ids, const gqm_cdt_in *in, gq
   if (grid < 1) return GQM_ERR_MEMORY;
   if (grow_dev(&C.d_in, &C.in_cap, in_bytes) || grow_dev(&C.d_out, &C.out_cap, out_bound) ||
       grow_dev(&C.d_arena, &C.arena_cap, arena * (size_t)grid) || grow_host(&C.h_in, &C.h_in_cap, in_bytes))
+    return GQM_ERR_MEMORY;
+  if (nb > 1 && (grow_dev(&C.d_teams, &C.teams_cap, sizeof(TeamState) * (size_t)grid) ||
+                 cudaMemsetAsync(C.d_teams, 0, sizeof(TeamState) * (size_t)grid, C.st) != cudaSuccess))
     return GQM_ERR_MEMORY;
   if (n > C.jobs_cap) {
     if (C.d_jobs) cudaFree(C.d_jobs);
@@ -940,10 +618,26 @@ int run_batch(DevCache &C, const std::vector<int> &ids, const gqm_cdt_in *in, gq
   const double h2d = ms_since(t0);
   // the persistent launch
   cudaEventRecord(C.e0, C.st);
+  TeamState *teams = reinterpret_cast<TeamState *>(C.d_teams);
 #ifdef GQM_HOST_EMU
-  V.fn(C.d_jobs, C.d_order, n, C.d_next, C.d_arena, arena, jobs[0].pred);
+  V.fn(C.d_jobs, C.d_order, n, C.d_next, C.d_arena, arena, teams, 1, jobs[0].pred);
 #else
-  V.fn<<<(unsigned)grid, V.threads, 0, C.st>>>(C.d_jobs, C.d_order, n, C.d_next, C.d_arena, arena, jobs[0].pred);
+  {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;  // blocks of a team wait for one another
+    at[0].val.cooperative = 1;
+    cfg.gridDim = dim3((unsigned)(grid * nb));
+    cfg.blockDim = dim3((unsigned)V.threads);
+    cfg.stream = C.st;
+    cfg.attrs = at;
+    cfg.numAttrs = nb > 1 ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, V.fn, C.d_jobs, (const int *)C.d_order, n, C.d_next, C.d_arena, arena, teams, nb,
+                           jobs[0].pred) != cudaSuccess) {
+      if (dnet) cudaFree(dnet);
+      return GQM_ERR_CUDA;
+    }
+  }
 #endif
   cudaEventRecord(C.e1, C.st);
   if (cudaStreamSynchronize(C.st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
@@ -1039,7 +733,7 @@ int run_batch(DevCache &C, const std::vector<int> &ids, const gqm_cdt_in *in, gq
       memcpy(R.tstatus, o + L.ts, (size_t)J.out_nt);
     });
   if (rep) {
-    rep->grid = (int)grid;
+    rep->grid = (int)(grid * nb);
     rep->threads_per_block = V.threads;
     rep->blocks_per_sm = V.minb;
     rep->arena_bytes = (long long)arena;
@@ -1143,6 +837,68 @@ int batch_call(int nd, const gqm_cdt_in *in, gqm_cdt_out *out, const gqm_options
 }  // namespace
 }  // namespace gqm
 
+// The refinement of one domain on the single-domain engine's buffers (refine.cu)
+// by one cooperative launch of `blocks` blocks.  scratch, caps, run and state
+// are the caller's Scratch, Caps, device EngineRun and device TeamState (the
+// same layouts in both compilations).
+int gqm_refine_one_launch(const void *scratch, size_t scratch_bytes, const void *caps, void *run, void *state, int pred,
+                          int blocks, int small_limit, void *ktimer, void *stimer, cudaStream_t st) {
+  using namespace gqm;
+  if (scratch_bytes != sizeof(Scratch)) return GQM_ERR_ARGUMENT;
+  Scratch S;
+  Caps c;
+  memcpy(&S, scratch, sizeof(S));
+  memcpy(&c, caps, sizeof(c));
+  EngineRun *r = static_cast<EngineRun *>(run);
+  TeamState *ts = static_cast<TeamState *>(state);
+  KTimer *kt = static_cast<KTimer *>(ktimer), *stm = static_cast<KTimer *>(stimer);
+#ifdef GQM_HOST_EMU
+  (void)blocks;
+  (void)st;
+  if (pred)
+    k_refine_one<1>(S, c, r, ts, small_limit, kt, stm);
+  else
+    k_refine_one<0>(S, c, r, ts, small_limit, kt, stm);
+  return GQM_OK;
+#else
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3(512);
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = pred ? cudaLaunchKernelEx(&cfg, k_refine_one<1>, S, c, r, ts, small_limit, kt, stm)
+                             : cudaLaunchKernelEx(&cfg, k_refine_one<0>, S, c, r, ts, small_limit, kt, stm);
+  return e == cudaSuccess ? GQM_OK : GQM_ERR_CUDA;
+#endif
+}
+// The incircle expansion-fallback counter of this translation unit's kernels
+// (see gqm_fallbacks_cluster in flipcl.cu).
+int gqm_fallbacks_cta(unsigned long long *sum, int reset, cudaStream_t st) {
+  unsigned long long v = 0;
+#ifdef GQM_HOST_EMU
+  (void)st;
+  v = gqm::g_incircle_fallbacks;
+  if (reset) gqm::g_incircle_fallbacks = 0;
+#else
+  if (sum && (cudaMemcpyFromSymbolAsync(&v, gqm::g_incircle_fallbacks, sizeof(v), 0, cudaMemcpyDeviceToHost, st) !=
+                  cudaSuccess ||
+              cudaStreamSynchronize(st) != cudaSuccess))
+    return GQM_ERR_CUDA;
+  if (reset) {
+    const unsigned long long zero = 0;
+    if (cudaMemcpyToSymbolAsync(gqm::g_incircle_fallbacks, &zero, sizeof(zero), 0, cudaMemcpyHostToDevice, st) !=
+        cudaSuccess)
+      return GQM_ERR_CUDA;
+  }
+#endif
+  if (sum) *sum += v;
+  return GQM_OK;
+}
+
 extern "C" {
 
 void gqm_default_batch_options(gqm_batch_options *b) {
@@ -1202,7 +958,7 @@ void gqm_batch_release(int device) {
   if (!C.init) return;
   cudaSetDevice(device);
   cudaStreamSynchronize(C.st);
-  void *dev[] = {C.d_in, C.d_out, C.d_arena, C.d_jobs, C.d_order, C.d_next, C.d_used};
+  void *dev[] = {C.d_in, C.d_out, C.d_arena, C.d_jobs, C.d_order, C.d_next, C.d_used, C.d_teams};
   for (void *p : dev)
     if (p) cudaFree(p);
   if (C.h_in) cudaFreeHost(C.h_in);
@@ -1211,8 +967,8 @@ void gqm_batch_release(int device) {
   cudaEventDestroy(C.e1);
   cudaStreamDestroy(C.st);
   const int tuned = C.tuned;
-  C.d_in = C.d_out = C.d_arena = C.h_in = C.h_out = nullptr;
-  C.in_cap = C.out_cap = C.arena_cap = C.h_in_cap = C.h_out_cap = 0;
+  C.d_in = C.d_out = C.d_arena = C.h_in = C.h_out = C.d_teams = nullptr;
+  C.in_cap = C.out_cap = C.arena_cap = C.h_in_cap = C.h_out_cap = C.teams_cap = 0;
   C.d_jobs = nullptr;
   C.d_order = nullptr;
   C.jobs_cap = 0;

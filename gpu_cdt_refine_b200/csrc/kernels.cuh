@@ -6,6 +6,7 @@
 #pragma once
 #include "gqm_device.cuh"
 #include "learned.cuh"
+#include "team.cuh"
 
 // Register budget of the latency-bound walk kernels (flip checks, cavity
 // walks, link updates): ask for at least this many resident 256-thread blocks
@@ -18,19 +19,18 @@
 //  * grid mode (default): every step below is a __global__ kernel whose
 //    grid-stride loop covers its items across the whole grid;
 //  * CTA mode (GQM_CTA_MODE, batch.cu): every step is a __device__ function
-//    that one thread block runs over one domain's items, the block's threads
-//    striding over them; the caller separates steps with __syncthreads();
-//  * cluster mode (GQM_CLUSTER_MODE, flipcl.cu): every step is a __device__
-//    function that the blocks of one thread-block cluster (the whole grid of
-//    the launch) run together, striding over the items with all their
-//    threads; the caller separates steps with cluster barriers.
+//    that a team of one or more thread blocks runs over one domain's items, the
+//    team's threads striding over them; the caller separates steps with the
+//    team's barrier (engine.cuh);
+//  * cluster mode (GQM_CLUSTER_MODE, flipcl.cu): the same with the whole grid
+//    as the team; of the steps below only the flip-flop loop is used there.
 #if defined(GQM_CTA_MODE)
 #define GQM_KERNEL __device__
 #define GQM_WALK_BOUNDS
 #define GQM_BOUNDS(minb)
-#define GQM_GTID ((int)threadIdx.x)
-#define GQM_GSIZE ((int)blockDim.x)
-#define GQM_BLOCK0 true
+#define GQM_GTID ((int)(gqm_team_rank * blockDim.x + threadIdx.x))
+#define GQM_GSIZE ((int)(gqm_team_blocks * blockDim.x))
+#define GQM_BLOCK0 (gqm_team_rank == 0)
 #elif defined(GQM_CLUSTER_MODE)
 #define GQM_KERNEL __device__
 #define GQM_WALK_BOUNDS
@@ -48,6 +48,11 @@
 #endif
 
 namespace gqm {
+
+#if defined(GQM_CTA_MODE)
+// the block's place in its team, and the team's blocks
+__shared__ int gqm_team_rank, gqm_team_blocks;
+#endif
 
 #define GS_LOOP(i, n) for (int i = GQM_GTID; i < (n); i += GQM_GSIZE)
 
@@ -345,6 +350,10 @@ GQM_KERNEL void k_mark_bad(Mesh M, N ntri_) {
 // ============================================================================
 __device__ __forceinline__ bool is_red(const Mesh &M, int p) { return M.pred[p] != 0; }
 
+// Generations that a loop (or a run's reset) advances by: the pushes for the
+// next loop carry its generation, and the claims that splitTriangles makes
+// before it carry the two before that.
+constexpr int kGenStride = 4, kGenLocate = 3, kGenCavity = 2;
 // Control block of the flip-flop loops, resident on the device.
 constexpr int kFlipProfileBins = 32;
 // List lengths of a flip step, indexed by the parity of the step's generation.
@@ -559,7 +568,7 @@ __device__ __forceinline__ void ctl_reset(FlipCtl *c, long long cap, int *errp, 
   if (!lead) return;
   for (int b = 0; b < kFlipProfileBins; ++b) c->prof_steps[b] = c->prof_items[b] = 0;
   c->cnt = FlipCnt{};
-  c->gen++;
+  c->gen += kGenStride;
   c->steps = 0;
   c->small_steps = 0;
   c->cap_hit = 0;
@@ -1108,7 +1117,6 @@ struct FlipRegs {
   int steps;
 };
 enum { FLIP_GO = 0, FLIP_DONE = 1, FLIP_BROKEN = 2 };
-__device__ __forceinline__ int vload(const int *p) { return *(const volatile int *)p; }
 template <int PRED, class Team>
 __device__ __forceinline__ int flip_step(const Mesh &M, const FlipLists &L, FlipCnt *cnt, FlipRegs &R, int entry_steps,
                                          Team &T, const int *cur, int n, int4 *rec, KTimer *tm, int *wins) {
@@ -1154,12 +1162,98 @@ __device__ __forceinline__ int flip_step(const Mesh &M, const FlipLists &L, Flip
   }
   return FLIP_GO;
 }
-// the loop's state back in the control block, ready for the next pushes
+// the loop's state back in the control block, ready for the next pushes (and the
+// claims of splitTriangles, which use the generations in between)
 __device__ __forceinline__ void flip_close(FlipCtl *c, const FlipRegs &R) {
   c->cnt = FlipCnt{};
-  c->gen = R.gen + 1;
+  c->gen = R.gen + kGenStride;
   c->epoch = R.epoch;
   c->steps = R.steps;
+}
+
+// shared-memory copies of the small steps' lists
+constexpr int kSmallCap = 1024;
+struct SmallLists {
+  FlipCnt cnt;
+  int4 rec[kSmallCap];
+};
+// One flip-flop loop (refine.cu:2328-2490) by the team G.  Most steps are
+// small: of the ~1,030 steps of a 2,000,000-point refinement, ~700 have at most
+// 1,024 queued triangles, and a barrier of all blocks would cost more than such
+// a step's work.  Those are run by the team's first block alone, whose barrier
+// is __syncthreads() and which keeps the list lengths and the decisions in
+// shared memory, or by the team S of the first few, while the other blocks wait
+// at one barrier.  ktm / stm: timers of the check phase of the steps run by all
+// blocks and of the small steps (probe), or null.  False when a barrier's wait
+// ran out.
+template <int PRED>
+__device__ __forceinline__ bool flip_loop(const Mesh &M, const FlipLists &L, SmallLists &sh, GridTeam &G, int small_limit,
+                                          GridTeam *S, KTimer *ktm, KTimer *stm) {
+  FlipCtl *c = L.c;
+  FlipRegs R{vload(&c->gen), (unsigned)vload((const int *)&c->epoch), vload(&c->steps)};
+  const int entry = R.steps;
+  const int timed = ktm ? ktm->on : 0;
+  const int small_blocks = S ? S->nb : 1;
+  const unsigned long long t0 = G.lead() ? global_ns() : 0;
+  int status = FLIP_GO;
+  // Every block takes the same way through the loop: what it decides on (list
+  // lengths, the control block) was written before the last barrier of all
+  // blocks and is not written again before the next.
+  while (status == FLIP_GO) {
+    const int n = vload(&c->cnt.qn[R.gen & 1]);
+    if (n == 0) break;
+    if (n > small_limit) {
+      status = flip_step<PRED>(M, L, &c->cnt, R, entry, G, (R.gen & 1) ? L.q1 : L.q0, n, L.rec, timed ? ktm : nullptr,
+                               nullptr);
+      continue;
+    }
+    const int steps0 = R.steps;
+    if (G.rank < small_blocks) {
+      const unsigned long long s0 = timed && G.lead() ? global_ns() : 0;
+      int items = 0, wins = 0, m = n;
+      if (!S) {
+        BlockTeam B;
+        if (B.lead()) sh.cnt = c->cnt;
+        B.sync();
+        while (status == FLIP_GO && m > 0 && m <= small_limit) {
+          items += m;
+          status = flip_step<PRED>(M, L, &sh.cnt, R, entry, B, (R.gen & 1) ? L.q1 : L.q0, m,
+                                   m <= kSmallCap ? sh.rec : L.rec, nullptr, timed ? &wins : nullptr);
+          m = vload(&sh.cnt.qn[R.gen & 1]);
+        }
+        B.sync();
+        if (B.lead()) c->cnt = sh.cnt;
+      } else {
+        while (status == FLIP_GO && m > 0 && m <= small_limit) {
+          items += m;
+          status = flip_step<PRED>(M, L, &c->cnt, R, entry, *S, (R.gen & 1) ? L.q1 : L.q0, m, L.rec, nullptr,
+                                   timed ? &wins : nullptr);
+          m = vload(&c->cnt.qn[R.gen & 1]);
+        }
+      }
+      if (G.lead()) {
+        c->gen = R.gen;
+        c->epoch = R.epoch;
+        c->steps = R.steps;
+        c->small_steps += R.steps - steps0;
+        c->small_status = status;
+        if (timed) ktimer_add(stm, s0, items, wins);
+      }
+    }
+    if (!G.sync()) return false;
+    R.gen = vload(&c->gen);
+    R.epoch = (unsigned)vload((const int *)&c->epoch);
+    R.steps = vload(&c->steps);
+    status = vload(&c->small_status);
+  }
+  if (status == FLIP_BROKEN || !G.sync()) return false;  // nobody reads the control block any more
+  if (G.lead()) {
+    flip_close(c, R);
+    c->ran++;
+    c->loop_ns += global_ns() - t0;
+    c->loops++;
+  }
+  return true;
 }
 
 // ============================================================================
@@ -1452,8 +1546,9 @@ GQM_KERNEL void k_circumcenter(Mesh M, const int *bad, const int *dn, double off
 
 // kernelLocateSinkPoints, refine.cu:3908-4184
 template <int PRED>
-GQM_KERNEL void k_locate(Mesh M, const int *bad, const int *dn, const double2 *center, int *sinks) {
+GQM_KERNEL void k_locate(Mesh M, const int *bad, const int *dn, const double2 *center, int *sinks, FlipLists L) {
   int n = *dn;
+  const int gen = L.c->gen - kGenLocate;
   GS_LOOP(k, n) {
     int index = bad[k];
     if (!(M.tst[index] & TS_BAD)) {
@@ -1534,28 +1629,29 @@ GQM_KERNEL void k_locate(Mesh M, const int *bad, const int *dn, const double2 *c
       curTri = dtri(nb);
       curOri = dori(nb);
     }
-    atomicMin(M.tmark + curTri, index);
+    claim(M, gen, curTri, index);
     if (split) {
       int nb = ld1(M.tn, curTri, dart);
-      if (nb != -1) atomicMin(M.tmark + dtri(nb), index);
+      if (nb != -1) claim(M, gen, dtri(nb), index);
     }
     sinks[k] = (curTri << 2) | dart;
   }
 }
 
 // kernelRemoveLosers, refine.cu:4186-4235
-GQM_KERNEL void k_remove_losers(Mesh M, const int *bad, const int *dn, const int *sinks, int *imark) {
+GQM_KERNEL void k_remove_losers(Mesh M, const int *bad, const int *dn, const int *sinks, int *imark, FlipLists L) {
   int n = *dn;
+  const int gen = L.c->gen - kGenLocate;
   GS_LOOP(k, n) {
     if (imark[k] < 0) continue;
     int sink = sinks[k] >> 2, dir = sinks[k] & 3, index = bad[k];
-    if (M.tmark[sink] != index) {
+    if (claimed(M, gen, sink) != index) {
       imark[k] = -1;
       continue;
     }
     if (dir != 3) {
       int nb = ld1(M.tn, sink, dir);
-      if (nb != -1 && M.tmark[dtri(nb)] != index) imark[k] = -1;
+      if (nb != -1 && claimed(M, gen, dtri(nb)) != index) imark[k] = -1;
     }
   }
 }
@@ -1587,7 +1683,7 @@ GQM_KERNEL void k_remove_losers(Mesh M, const int *bad, const int *dn, const int
 // the same edges as one that tests each neighbour when it gets to it.
 __device__ __forceinline__ unsigned cavity_hash(int t) { return ((unsigned)t * 2654435761u) >> 26; }
 template <int PRED>
-__device__ int cavity_walk(const Mesh &M, int sink, int direction, double2 cc, int badIndex, int *out,
+__device__ int cavity_walk(const Mesh &M, int gen, int sink, int direction, double2 cc, int badIndex, int *out,
                            int stride) {
   int region[kCavityCap], loop[kCavityCap];  // loop: (triangle << 2) | edge to resume at
   uint8_t inside[kCavityCap];                // per frame: neighbours whose circumcircle holds cc
@@ -1603,7 +1699,7 @@ __device__ int cavity_walk(const Mesh &M, int sink, int direction, double2 cc, i
       region[rsize++] = cur;
       rbits |= 1ull << cavity_hash(cur);
       loop[lsize++] = cur << 2;
-      atomicMin(M.tmark + cur, badIndex);
+      claim(M, gen, cur, badIndex);
       const int4 sg = M.tsg[cur];
       nb = M.tn[cur];
       int tt[3];
@@ -1671,12 +1767,13 @@ __device__ int cavity_walk(const Mesh &M, int sink, int direction, double2 cc, i
 // index).  cavn[k] = stored cavity size (0 for an oversized one).
 template <int PRED>
 GQM_KERNEL void GQM_WALK_BOUNDS k_cavity_mark(Mesh M, const int *dn, const int *sinks, const double2 *center, const int *imark,
-                              int *ilist, int *cav, int *cavn, int stride) {
+                              int *ilist, int *cav, int *cavn, int stride, FlipLists L) {
   int n = *dn;
+  const int gen = L.c->gen - kGenCavity;
   GS_LOOP(k, n) {
     if (imark[k] < 0) continue;
     int badIndex = ilist[k];
-    int c = cavity_walk<PRED>(M, sinks[k] >> 2, sinks[k] & 3, center[k], badIndex, cav + k, stride);
+    int c = cavity_walk<PRED>(M, gen, sinks[k] >> 2, sinks[k] & 3, center[k], badIndex, cav + k, stride);
     if (c < 0) ilist[k] = negate_idx(badIndex);
     cavn[k] = c < 0 ? 0 : c;
   }
@@ -1684,15 +1781,16 @@ GQM_KERNEL void GQM_WALK_BOUNDS k_cavity_mark(Mesh M, const int *dn, const int *
 // kernelCheckCavities: a candidate loses if any triangle of its cavity was
 // claimed by a smaller bad index.
 GQM_KERNEL void k_cavity_check(Mesh M, const int *dn, const int *cav, const int *cavn, int stride, int *imark,
-                               const int *ilist) {
+                               const int *ilist, FlipLists L) {
   int n = *dn;
+  const int gen = L.c->gen - kGenCavity;
   GS_LOOP(k, n) {
     if (imark[k] < 0) continue;
     int badIndex = ilist[k];
     if (badIndex < 0) continue;
     int c = cavn[k];
     for (int j = 0; j < c; ++j)
-      if (M.tmark[cav[(long)j * stride + k]] != badIndex) {
+      if (claimed(M, gen, cav[(long)j * stride + k]) != badIndex) {
         imark[k] = -1;
         break;
       }
@@ -1953,8 +2051,8 @@ GQM_KERNEL void k_emit_pstatus(Mesh M, int np, uint8_t *pstat) {
 // The placement step and the collection of training data
 // ---------------------------------------------------------------------------
 #ifdef GQM_CTA_MODE
-#define GQM_BID 0
-#define GQM_NB 1
+#define GQM_BID gqm_team_rank
+#define GQM_NB gqm_team_blocks
 #else
 #define GQM_BID ((int)blockIdx.x)
 #define GQM_NB ((int)gridDim.x)

@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -24,7 +25,7 @@
 
 #include "../../include/gqm_refine.h"
 #include "host_copy.h"
-#include "kernels.cuh"
+#include "engine.cuh"
 
 // NVTX ranges around the driver's phases (refinement, encroached-subsegment
 // splitting, Steiner rounds, flip-flop loops, output compaction, result
@@ -50,7 +51,11 @@ int gqm_flip_max_blocks(int budget);
 int gqm_flip_loop_launch(const void *mesh, size_t mesh_bytes, const void *lists, size_t lists_bytes, void *bars,
                          const int *team, int pred, int blocks, int budget, int small_limit, int small_team,
                          void *ktimer, void *stimer, cudaStream_t st);
-// the incircle expansion-fallback counter of flipcl.cu's kernels
+// batch.cu: the whole refinement of one domain in one cooperative launch
+int gqm_refine_one_launch(const void *scratch, size_t scratch_bytes, const void *caps, void *run, void *state, int pred,
+                          int blocks, int small_limit, void *ktimer, void *stimer, cudaStream_t st);
+// the incircle expansion-fallback counters of batch.cu's and flipcl.cu's kernels
+int gqm_fallbacks_cta(unsigned long long *sum, int reset, cudaStream_t st);
 int gqm_fallbacks_cluster(unsigned long long *sum, int reset, cudaStream_t st);
 
 namespace gqm {
@@ -276,6 +281,13 @@ __global__ void k_set_count(int *dst, int v) {
 // subsegments and the round loop, refine.cu:6830-7024) runs as one CUDA graph
 // whose loops and branches are conditional nodes decided on the device.
 // ============================================================================
+// Largest input of the one-launch refinement (triangles).  The emulated build
+// of the tests takes it for the smaller half of its inputs.
+#ifdef GQM_HOST_EMU
+#define GQM_ONE_LAUNCH_TRIS 4000
+#else
+#define GQM_ONE_LAUNCH_TRIS (1 << 20)
+#endif
 constexpr int kMaxNodes = 40;  // conditional nodes of the refinement graph
 struct DState {
   int pcap, tcap;                  // the reference's logical capacities of points / triangles
@@ -639,7 +651,9 @@ struct Refiner {
   int *cav = nullptr, *cavn = nullptr;  // stored cavities of the Steiner candidates
   long cav_cap = 0;
   FlipLists fl{};         // lists of the flip steps, and their control block (device)
-  FlipCtl *fc = nullptr;  // = fl.c
+  FlipCtl *fc = nullptr;  // = fl.c, in team
+  TeamState *team = nullptr;  // state of the one-launch refinement
+  EngineRun *run_d = nullptr;
   char *bars = nullptr;   // barrier words of the flip loop's launch
   KTimer *ktm = nullptr;  // timer of the check phase of the steps run by all blocks
   KTimer *stm = nullptr;  // timer of the small steps
@@ -755,7 +769,7 @@ struct Refiner {
     void *ptrs[] = {M.pts, M.ps, M.pred, M.tv, M.tn, M.tsg, M.tst, M.tflip, M.tfo, M.tmark, M.fmark, M.emap,
                     M.s2t, M.s2seg, M.enc, M.err, stm, emptyt, bad, imark, ilist, sinks, wl,
                     newidx, tail, center, emptyp, pnew, enclist, encl2, smark, mids, snap, segs, dcount, bc,
-                    dctr, dgc, dinput, mlp_w, mlp_b, M.fstamp, fl.q0, fl.q1, fl.rec, fl.red, fl.late, fl.wbits, fc, cav, cavn, ktm, bars, ds, csync};
+                    dctr, dgc, dinput, mlp_w, mlp_b, M.fstamp, fl.q0, fl.q1, fl.rec, fl.red, fl.late, fl.wbits, team, run_d, cav, cavn, ktm, bars, ds, csync};
     for (void *p : ptrs)
       if (p) cudaFree(p);
     if (hcount) cudaFreeHost(hcount);
@@ -764,6 +778,8 @@ struct Refiner {
     emptyt = bad = imark = ilist = sinks = wl = newidx = tail = nullptr;
     fl = FlipLists{};
     fc = nullptr;
+    team = nullptr;
+    run_d = nullptr;
     bars = nullptr;
     ktm = nullptr;
     stm = nullptr;
@@ -810,12 +826,13 @@ struct Refiner {
       if (loop_blocks[b] <= 0 && (loop_blocks[b] = gqm_flip_max_blocks(b)) <= 0) return GQM_ERR_CUDA;
     if (!dcount) {
       if (dalloc(&dcount, 16) || dalloc(&bc, kMaxCompactBlocks + 1) || dalloc(&dctr, 8) || dalloc(&dgc, 2) ||
-          dalloc(&M.err, 1) || dalloc(&fc, 1) || dalloc(&ktm, 1) || dalloc(&stm, 1) || dalloc(&ds, 1) ||
+          dalloc(&M.err, 1) || dalloc(&team, 1) || dalloc(&run_d, 1) || dalloc(&ktm, 1) || dalloc(&stm, 1) || dalloc(&ds, 1) ||
           dalloc(&csync, 1) || dalloc(&bars, gqm_flip_bar_bytes()))
         return GQM_ERR_MEMORY;
+      fc = &team->fc;
       fl.c = fc;
       cudaMemsetAsync(csync, 0, sizeof(CompactSync), st);
-      cudaMemsetAsync(fc, 0, sizeof(FlipCtl), st);
+      cudaMemsetAsync(team, 0, sizeof(TeamState), st);
       cudaMemsetAsync(ktm, 0, sizeof(KTimer), st);  // off until gqm_context_probe
       cudaMemsetAsync(stm, 0, sizeof(KTimer), st);
       cudaMemsetAsync(bc + kMaxCompactBlocks, 0, sizeof(int), st);  // the zero base of one-block compactions
@@ -824,6 +841,7 @@ struct Refiner {
 #else
       const char *ng = getenv("GQM_NO_GRAPH");
       use_graph = !(ng && ng[0] == '1');
+      one_launch_ok = use_graph;
 #endif
       if (cudaMallocHost((void **)&hcount, sizeof(int) * 16) != cudaSuccess) return GQM_ERR_MEMORY;
     }
@@ -1125,7 +1143,7 @@ struct Refiner {
   // Launch shape of the flip-flop loop (gqm_tuning).  None of it changes a
   // result: every step makes the reference's decisions whatever the grid.
 #ifndef GQM_SMALL_STEP
-#define GQM_SMALL_STEP 1024
+#define GQM_SMALL_STEP 256
 #endif
   struct Tuning {
     int step_grid = 148 * 4;           // most blocks of a step (beyond one per SM: one per SM)
@@ -1147,12 +1165,17 @@ struct Refiner {
                                 loop_blocks[tune.check_minb], tune.check_minb, tune.small_limit, tune.small_cluster,
                                 ktm, stm, st);
   }
-  // Blocks that a refinement's flip loops use: one per 1,024 input triangles,
-  // at most one per SM (or step_grid).  A step's barriers cost more the more
-  // blocks take part, and a small input's steps never fill a large team.
+  // Blocks that a refinement uses.  A barrier of several blocks costs several
+  // times that of one, and the largest inputs' steps fill every SM: 980
+  // triangles (500 points) take 2.8 ms with one block and 3.6 ms with 16, 6,000
+  // triangles 12.2, 11.0 and 10.9 ms with 1, 8 and 16, 20,000 triangles 10.8,
+  // 10.6 and 10.8 ms with 16, 32 and 148, 60,000 triangles 15.6, 15.2 and
+  // 15.4 ms with 32, 64 and 148, 200,000 triangles 20.1 and 19.6 ms with 64
+  // and 148 (steps of up to 512 triangles by the first block).
   int team_blocks(int nt) const {
+    if (nt <= 2048) return 1;
     const int most = std::min(tune.step_grid, loop_blocks[tune.check_minb]);
-    return std::max(1, std::min(most, (nt + 1023) / 1024));
+    return std::max(1, std::min(most, std::max(16, nt / 512)));
   }
 
   // ---- splitEncsegs (refine.cu:3180-3778) ----
@@ -1217,19 +1240,17 @@ struct Refiner {
       KL(k_learned_place, kDevGrid, 32 * kInferWarpsMax)(M, bad, dn, mlp_dev(mlp_w, mlp_b), center, dctr + 4);
       count_launch(1);
     }
-    DLAUNCH(k_fill_n, M.tmark, DevInt{&ds->last_triangle}, kMaxInt);
     if (pred_mode)
-      DLAUNCH(k_locate<1>, M, bad, dn, center, sinks);
+      DLAUNCH(k_locate<1>, M, bad, dn, center, sinks, fl);
     else
-      DLAUNCH(k_locate<0>, M, bad, dn, center, sinks);
-    DLAUNCH(k_remove_losers, M, bad, dn, sinks, imark);
-    DLAUNCH(k_fill_n, M.tmark, DevInt{&ds->last_triangle}, kMaxInt);
+      DLAUNCH(k_locate<0>, M, bad, dn, center, sinks, fl);
+    DLAUNCH(k_remove_losers, M, bad, dn, sinks, imark, fl);
     // stored cavities: kCavityCap rows of cav_cap entries
     if (pred_mode)
-      DLAUNCH(k_cavity_mark<1>, M, dn, sinks, center, imark, ilist, cav, cavn, (int)cav_cap);
+      DLAUNCH(k_cavity_mark<1>, M, dn, sinks, center, imark, ilist, cav, cavn, (int)cav_cap, fl);
     else
-      DLAUNCH(k_cavity_mark<0>, M, dn, sinks, center, imark, ilist, cav, cavn, (int)cav_cap);
-    DLAUNCH(k_cavity_check, M, dn, cav, cavn, (int)cav_cap, imark, ilist);
+      DLAUNCH(k_cavity_mark<0>, M, dn, sinks, center, imark, ilist, cav, cavn, (int)cav_cap, fl);
+    DLAUNCH(k_cavity_check, M, dn, cav, cavn, (int)cav_cap, imark, ilist, fl);
     compact_dev(PNonNeg{imark}, Ident{}, dn, wl, &ds->nst);
     DLAUNCH(k_fill_n, encl2, DevInt{&ds->last_subseg}, -1);
     DLAUNCH(k_mark_onsegs, M, wl, &ds->nst, sinks, encl2);
@@ -1420,6 +1441,116 @@ struct Refiner {
     return GQM_OK;
   }
 
+  void grow_buffers(int need) {
+    if (need & 1) want_p = 2 * pphys;
+    if (need & 2) want_t = 2 * tphys;
+    if (need & 4) want_s = 2 * sphys;
+    if (need & 8) want_cav = 2 * cav_cap;
+  }
+
+  // ---- the refinement in one cooperative launch (engine.cuh) ----
+  // Up to kOneLaunchTris input triangles the launches, condition nodes and
+  // fixed grids of the graph cost more than a barrier of the team between two
+  // steps; beyond, the passes over all triangles want more warps than the
+  // launch's registers leave.  Device time with the graph and in one launch:
+  // 500 points 4.3 and 2.7 ms, 3,000 points 12.2 and 10.9 ms, 100,000 points
+  // 21.2 and 19.3 ms, 500,000 points 33.1 and 32.0 ms, 700,000 points 38.3 and
+  // 38.3 ms, 1,000,000 points 52.6 and 54.4 ms.
+  static constexpr int kOneLaunchTris = GQM_ONE_LAUNCH_TRIS;
+  bool one_launch_ok = true;
+  bool one_launch(int nt) const { return one_launch_ok && !explore && !col_feat && nt <= kOneLaunchTris; }
+  EngineRun hrun{};
+  int run_one_launch(const gqm_options *opt, const double *dpts, const int *dtri, const int *dnbr, int np, int nt,
+                     int ns, unsigned hsz) {
+    Scratch S{};
+    S.M = M;
+    S.emptyt = emptyt;
+    S.bad = bad;
+    S.imark = imark;
+    S.ilist = ilist;
+    S.sinks = sinks;
+    S.wl = wl;
+    S.newidx = newidx;
+    S.tail = tail;
+    S.emptyp = emptyp;
+    S.pnew = pnew;
+    S.enclist = enclist;
+    S.encl2 = encl2;
+    S.smark = smark;
+    S.mids = mids;
+    S.snap = snap;
+    S.cav = cav;
+    S.cavn = cavn;
+    S.fl = fl;
+    S.center = center;
+    S.hkeys = hkeys;
+    S.hvals = hvals;
+    S.s2ti = s2ti;
+    const Caps c{pointblock, triblock, pphys, tphys, sphys, cav_cap, (long)hsz};
+    hrun = EngineRun{};
+    hrun.pts = reinterpret_cast<const double2 *>(dpts);
+    hrun.tri = dtri;
+    hrun.nbr = dnbr;
+    hrun.seg = segs;
+    hrun.np = np;
+    hrun.nt = nt;
+    hrun.ns = ns;
+    hrun.offcenter = offcenter;
+    hrun.offconstant = offconstant;
+    hrun.mode = mode;
+    hrun.pred = pred_mode;
+    hrun.placement = placement;
+    if (placement == GQM_PLACE_LEARNED) hrun.mlp = mlp_dev(mlp_w, mlp_b);
+    hrun.theta = theta;
+    hrun.max_area = opt->max_area > 0.0 ? opt->max_area : 0.0;
+    hrun.max_rounds = max_rounds;
+    cudaMemcpyAsync(run_d, &hrun, sizeof(EngineRun), cudaMemcpyHostToDevice, st);
+    // the team's state afresh, but for the control block's generation and epoch
+    cudaMemsetAsync(&team->bar, 0, sizeof(TeamState) - offsetof(TeamState, bar), st);
+    KL(k_ctl_reset, 1, 32)(fc, 64 * max_rounds, &team->err);
+    gqm_fallbacks_cta(nullptr, 1, st);
+    int rc = gqm_refine_one_launch(&S, sizeof(S), &c, run_d, team, pred_mode, team_blocks(nt), tune.small_limit, ktm,
+                                   stm, st);
+    if (rc) return rc;
+    cudaEventRecord(ev1, st);
+    cudaMemcpyAsync(&hrun, run_d, sizeof(EngineRun), cudaMemcpyDeviceToHost, st);
+    FlipCtl hf;
+    cudaMemcpyAsync(&hf, fc, sizeof(hf), cudaMemcpyDeviceToHost, st);
+    unsigned long long fb = 0;
+    rc = gqm_fallbacks_cta(&fb, 0, st);  // synchronises
+    if (rc) return rc;
+    if (hrun.status == GQM_ERR_ARENA) return hrun.need_grow ? GQM_OK : GQM_ERR_MEMORY;  // repeated with larger buffers
+    hrun.need_grow = 0;
+    M.gc2 = hrun.goodcos2;
+    M.mode = mode;
+    M.max_area = hrun.max_area;
+    last_point = hrun.last_point;
+    last_triangle = hrun.last_triangle;
+    last_subseg = hrun.out_ns;
+    out_np = hrun.out_np;
+    out_nt = hrun.out_nt;
+    out_ns = hrun.out_ns;
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ev0, ev1);
+    stats.device_ms = ms;
+    stats.goodcos2 = hrun.goodcos2;
+    stats.rounds = hrun.rounds;
+    stats.bad_total = hrun.bad_total;
+    stats.kernel_launches = 2;
+    stats.host_syncs = 1;
+    stats.steiner_inserted = (long long)hrun.ctr[0];
+    stats.midpoints_inserted = (long long)hrun.ctr[1];
+    stats.learned_candidates = (long long)hrun.ctr[4];
+    stats.learned_used = (long long)hrun.ctr[5];
+    stats.exact_fallbacks = (long long)fb;
+    stats.flip_steps = hf.steps;
+    for (int b = 0; b < kFlipProfileBins; ++b) {
+      flip_prof_steps[b] = (long long)hf.prof_steps[b];
+      flip_prof_items[b] = (long long)hf.prof_items[b];
+    }
+    return hrun.status;
+  }
+
   // ---- the whole refinement ----
   int run(const gqm_cdt_in *in, bool on_device, const gqm_options *opt) {
     NvtxRange nvtx("gqm:refine");
@@ -1526,6 +1657,31 @@ struct Refiner {
     if (grow_dev(&segs, &segs_cap, (size_t)ns + 1)) return GQM_ERR_MEMORY;
     if (ns) cudaMemcpyAsync(segs, dseg_in, sizeof(int2) * ns, cudaMemcpyDeviceToDevice, st);
     M.segs = segs;
+    // initSubsegs' hash of segment endpoints
+    unsigned hsz = 1;
+    while (hsz < 2u * (unsigned)ns + 16) hsz <<= 1;
+    if (hsz > hash_cap) {  // the three tables share one capacity, set once all three exist
+      hash_cap = 0;
+      size_t c0 = 0, c1 = 0, c2 = 0;
+      if (hvals) cudaFree(hvals);
+      if (s2ti) cudaFree(s2ti);
+      hvals = nullptr;
+      s2ti = nullptr;
+      if (grow_dev(&hkeys, &c0, hsz) || grow_dev(&hvals, &c1, hsz) || grow_dev(&s2ti, &c2, hsz))
+        return GQM_ERR_MEMORY;
+      hash_cap = hsz;
+    }
+    if (one_launch(nt)) {
+      rc = run_one_launch(opt, dpts, dtri_in, dnbr_in, np, nt, ns, hsz);
+      if (rc == GQM_OK && hrun.need_grow) {
+        if (++attempt > 8) return GQM_ERR_MEMORY;
+        grow_buffers(hrun.need_grow);
+        goto restart;
+      }
+      have_result = rc == GQM_OK;
+      status = rc;
+      return rc;
+    }
     cudaMemsetAsync(M.s2t, 0, sizeof(s2t_t) * sphys, st);
     cudaMemsetAsync(bars, 0, gqm_flip_bar_bytes(), st);
     cudaMemsetAsync(M.err, 0, sizeof(int), st);
@@ -1551,26 +1707,11 @@ struct Refiner {
     LAUNCH(k_init_points, pphys, M, (const double2 *)dpts, np, (int)pphys);
     LAUNCH(k_init_tris, tphys, M, dtri_in, dnbr_in, nt, (int)tphys);
     // initSubsegs via a hash of segment endpoints
-    {
-      unsigned hsz = 1;
-      while (hsz < 2u * (unsigned)ns + 16) hsz <<= 1;
-      if (hsz > hash_cap) {  // the three tables share one capacity, set once all three exist
-        hash_cap = 0;
-        size_t c0 = 0, c1 = 0, c2 = 0;
-        if (hvals) cudaFree(hvals);
-        if (s2ti) cudaFree(s2ti);
-        hvals = nullptr;
-        s2ti = nullptr;
-        if (grow_dev(&hkeys, &c0, hsz) || grow_dev(&hvals, &c1, hsz) || grow_dev(&s2ti, &c2, hsz))
-          return GQM_ERR_MEMORY;
-        hash_cap = hsz;
-      }
-      cudaMemsetAsync(hkeys, 0xff, sizeof(unsigned long long) * hsz, st);
-      cudaMemsetAsync(s2ti, 0xff, sizeof(int) * (ns + 1), st);
-      LAUNCH(k_seg_hash_insert, ns, segs, ns, hkeys, hvals, hsz - 1);
-      LAUNCH(k_init_subsegs, nt, M, nt, hkeys, hvals, hsz - 1, s2ti);
-      LAUNCH(k_pack_s2t, ns, M, s2ti, ns);
-    }
+    cudaMemsetAsync(hkeys, 0xff, sizeof(unsigned long long) * hsz, st);
+    cudaMemsetAsync(s2ti, 0xff, sizeof(int) * (ns + 1), st);
+    LAUNCH(k_seg_hash_insert, ns, segs, ns, hkeys, hvals, hsz - 1);
+    LAUNCH(k_init_subsegs, nt, M, nt, hkeys, hvals, hsz - 1, s2ti);
+    LAUNCH(k_pack_s2t, ns, M, s2ti, ns);
     // the driver's state on the device: the reference's logical capacities
     // and high-water marks, and the physical capacities a run must stay in
     hds = DState{};
@@ -1598,10 +1739,7 @@ struct Refiner {
       // a physical capacity would have been exceeded: repeat the run with
       // larger buffers (the result does not depend on them)
       if (++attempt > 8) return GQM_ERR_MEMORY;
-      if (hds.need_grow & 1) want_p = 2 * pphys;
-      if (hds.need_grow & 2) want_t = 2 * tphys;
-      if (hds.need_grow & 4) want_s = 2 * sphys;
-      if (hds.need_grow & 8) want_cav = 2 * cav_cap;
+      grow_buffers(hds.need_grow);
       pcap = np + pointblock;
       tcap = nt + triblock;
       stats = gqm_stats{};
@@ -1867,7 +2005,7 @@ int gqm_context_autotune(gqm_context *ctx, const gqm_cdt_in *in, int in_on_devic
   // device cannot run (a cluster size it cannot place) is skipped
   const int checks[] = {2, 1};
   const int clusters[] = {1, 8, 16};
-  const int limits[] = {512, 1024, 2048, 4096};
+  const int limits[] = {128, 256, 512, 1024};
   const int grids[] = {148 * 2, 148 * 4, 148 * 8};
   for (int field = 0; field < 4; ++field) {
     const int *vals = field == 0 ? checks : field == 1 ? clusters : field == 2 ? limits : grids;

@@ -166,10 +166,10 @@ void *gqm_context_stream(gqm_context *ctx);
  * result: every flip step makes the reference's decisions whatever the launch
  * shape.  Zero in a field means its default. */
 typedef struct {
-  int step_grid;           /* most blocks of a flip step (default 592; never more than one per SM, nor than
-                              one per 1,024 input triangles) */
+  int step_grid;           /* most blocks of a flip step (default 592; never more than one per SM, nor more
+                              than the input's size asks for) */
   int small_limit;         /* flip steps of at most this many queued triangles are run by the small team
-                              (default 1024; negative: never) */
+                              (default 256; negative: never) */
   int small_cluster;       /* blocks of the small team: 1 (default; its lists in shared memory), 8 or 16 */
   int check_blocks_per_sm; /* register budget of the flip loop: 2 = 512 threads per SM at most 128 registers
                               each (default), 1 = 256 threads at up to 255 */
@@ -232,9 +232,10 @@ int gqm_refine_batch(int ndomains, const gqm_cdt_in *in, gqm_cdt_out *out, const
 
 /* Persistent batched refinement (no counterpart in the reference, which
  * refines one CDT per call).  One kernel launch refines every domain: each
- * thread block takes the next domain from a queue ordered largest first and
- * runs the whole refinement of it (rounds, flip-flop loops, compaction) on the
- * device, in a scratch arena of its own sized for the largest domain.  Each
+ * team of thread blocks (one block in a large batch, several where domains are
+ * few) takes the next domain from a queue ordered largest first and runs the
+ * whole refinement of it (rounds, flip-flop loops, compaction) on the device, in
+ * a scratch arena of its own sized for the largest domain.  Each
  * domain's result is the one gqm_refine would return for it.  A domain whose
  * mesh outgrows its arena (GQM_ERR_ARENA) is refined again by the
  * single-domain GPU path; report->fallbacks counts those.  All domains must
