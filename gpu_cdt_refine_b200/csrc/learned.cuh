@@ -14,7 +14,7 @@
 //
 // The network: 32 fp32 features -> 64 -> 64 -> 1, ReLU, weights in bf16, fp32
 // accumulation on the tensor cores (mma.sync m16n8k16, bf16 x bf16 -> fp32),
-// biases in fp32.  The same warp-level GEMM serves inference and training.
+// biases in fp32.
 #pragma once
 #include <cstdint>
 
@@ -60,88 +60,8 @@ inline void mlp_pack(const float *params, uint16_t *w, float *b) {
   b[2 * kHid] = params[kOffB3];
 }
 
-// ---------------------------------------------------------------------------
-// Warp GEMM on shared-memory operands: C[i][j] (+)= sum_k A(i,k) B(k,j) with
-// A(i,k) = a[i*ai + k*ak], B(k,j) = b[k*bk + j*bj] (bf16 bits), M % 16 == 0,
-// N % 8 == 0, K % 16 == 0; C(i,j) = c[i*ci + j*cj] in fp32.  Called by all 32
-// lanes of a warp.  Fragment layout of mma.m16n8k16 (PTX ISA): lane = 4 g + q;
-// A regs (g, 2q..2q+1), (g+8, 2q..), (g, 2q+8..), (g+8, 2q+8..); B regs
-// (2q..2q+1, g), (2q+8.., g); C (g, 2q..2q+1), (g+8, 2q..2q+1).
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack2(uint16_t lo, uint16_t hi) { return (uint32_t)lo | ((uint32_t)hi << 16); }
-__device__ inline void warp_gemm(int M, int N, int K, const uint16_t *a, int ai, int ak, const uint16_t *b, int bk,
-                                 int bj, float *c, int ci, int cj, bool accumulate) {
-#ifdef GQM_HOST_EMU
-  for (int i = 0; i < M; ++i)
-    for (int j = 0; j < N; ++j) {
-      float s = accumulate ? c[i * ci + j * cj] : 0.0f;
-      for (int k = 0; k < K; ++k) s += bf2f(a[i * ai + k * ak]) * bf2f(b[k * bk + j * bj]);
-      c[i * ci + j * cj] = s;
-    }
-#else
-  const int lane = (int)(threadIdx.x & 31u), g = lane >> 2, q = lane & 3;
-  for (int i0 = 0; i0 < M; i0 += 16)
-    for (int j0 = 0; j0 < N; j0 += 8) {
-      float d[4];
-      d[0] = accumulate ? c[(i0 + g) * ci + (j0 + 2 * q) * cj] : 0.0f;
-      d[1] = accumulate ? c[(i0 + g) * ci + (j0 + 2 * q + 1) * cj] : 0.0f;
-      d[2] = accumulate ? c[(i0 + g + 8) * ci + (j0 + 2 * q) * cj] : 0.0f;
-      d[3] = accumulate ? c[(i0 + g + 8) * ci + (j0 + 2 * q + 1) * cj] : 0.0f;
-      for (int k0 = 0; k0 < K; k0 += 16) {
-        const uint16_t *A = a + i0 * ai + k0 * ak;
-        const uint16_t *B = b + k0 * bk + j0 * bj;
-        uint32_t ra[4], rb[2];
-        ra[0] = pack2(A[g * ai + (2 * q) * ak], A[g * ai + (2 * q + 1) * ak]);
-        ra[1] = pack2(A[(g + 8) * ai + (2 * q) * ak], A[(g + 8) * ai + (2 * q + 1) * ak]);
-        ra[2] = pack2(A[g * ai + (2 * q + 8) * ak], A[g * ai + (2 * q + 9) * ak]);
-        ra[3] = pack2(A[(g + 8) * ai + (2 * q + 8) * ak], A[(g + 8) * ai + (2 * q + 9) * ak]);
-        rb[0] = pack2(B[(2 * q) * bk + g * bj], B[(2 * q + 1) * bk + g * bj]);
-        rb[1] = pack2(B[(2 * q + 8) * bk + g * bj], B[(2 * q + 9) * bk + g * bj]);
-        asm volatile(
-            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-            "{%0,%1,%2,%3};\n"
-            : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-            : "r"(ra[0]), "r"(ra[1]), "r"(ra[2]), "r"(ra[3]), "r"(rb[0]), "r"(rb[1]));
-      }
-      __syncwarp();
-      c[(i0 + g) * ci + (j0 + 2 * q) * cj] = d[0];
-      c[(i0 + g) * ci + (j0 + 2 * q + 1) * cj] = d[1];
-      c[(i0 + g + 8) * ci + (j0 + 2 * q) * cj] = d[2];
-      c[(i0 + g + 8) * ci + (j0 + 2 * q + 1) * cj] = d[3];
-      __syncwarp();
-    }
-#endif
-}
-
-// Forward pass of 32 rows (row r = lane r) held in x (bf16, 32 x 32) in shared
-// memory; h (fp32, 32 x 64) and a1 (bf16, 32 x 64) are shared scratch, a2
-// (bf16, 32 x 64) keeps the second layer's activations when not null.
-// Returns this lane's output.  Weights are read from global memory (bf16).
-__device__ inline float mlp_forward_warp(const MlpDev &P, const uint16_t *x, float *h, uint16_t *a1, uint16_t *a2) {
-  const int lane = (int)(threadIdx.x & 31u);
-  __syncwarp();
-  // layer 1: h = x W1^T
-  warp_gemm(32, kHid, kFeat, x, kFeat, 1, P.w1, 1, kFeat, h, kHid, 1, false);
-  __syncwarp();
-  for (int j = 0; j < kHid; ++j) {
-    const float v = h[lane * kHid + j] + P.b1[j];
-    a1[lane * kHid + j] = f2bf(v > 0.0f ? v : 0.0f);
-  }
-  __syncwarp();
-  // layer 2: h = a1 W2^T
-  warp_gemm(32, kHid, kHid, a1, kHid, 1, P.w2, 1, kHid, h, kHid, 1, false);
-  __syncwarp();
-  float y = P.b3[0];
-  for (int j = 0; j < kHid; ++j) {
-    const float v = h[lane * kHid + j] + P.b2[j];
-    const uint16_t hb = f2bf(v > 0.0f ? v : 0.0f);
-    if (a2) a2[lane * kHid + j] = hb;
-    y += bf2f(hb) * bf2f(P.w3[j]);
-  }
-  __syncwarp();
-  return y;
-}
-// The same network for one row with scalar arithmetic (the CPU emulation of
+// The network for one row with scalar arithmetic (the CPU emulation of
 // the tests runs kernels one thread at a time, without warps).
 __host__ __device__ inline float mlp_forward_row(const MlpDev &P, const float *f) {
   float a1[kHid], y = P.b3[0];
@@ -159,20 +79,13 @@ __host__ __device__ inline float mlp_forward_row(const MlpDev &P, const float *f
   }
   return y;
 }
-struct MlpInferSmem {
-  uint16_t x[32 * kFeat];
-  float h[32 * kHid];
-  uint16_t a1[32 * kHid];
-};
-
 // ---------------------------------------------------------------------------
 // Inference with the weights staged in shared memory once per block and the
 // activations kept in registers: the accumulator fragments of two adjacent
 // 8-column tiles of one layer are, after bias, ReLU and bf16 rounding, the A
-// fragment of a 16-column step of the next layer (mma.m16n8k16 layouts, as in
-// warp_gemm above).  Rows of the weight and input tiles are padded by 8 bf16
+// fragment of a 16-column step of the next layer.  Rows of the weight and input tiles are padded by 8 bf16
 // so that the fragment loads of a warp hit 32 distinct banks.  Layers 1 and 2
-// round exactly as mlp_forward_warp; layer 3 sums a lane's 16 columns and then
+// round exactly as training does; layer 3 sums a lane's 16 columns and then
 // the four lanes of a quad, so its fp32 rounding order differs from the
 // sequential sum there.
 // ---------------------------------------------------------------------------
