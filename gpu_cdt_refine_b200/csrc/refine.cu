@@ -1155,6 +1155,7 @@ struct Refiner {
              check_minb == o.check_minb;
     }
   } tune;
+  int sharers = 1;  // contexts that run on the device at the same time: each takes its part of the SMs
   int loop_blocks[3] = {0, 0, 0};  // most resident blocks of the loop's launch, by register budget (0: not asked yet)
 
   // ---- flip-flop (refine.cu:2328-2490) over the triangles flagged since the last loop ----
@@ -1162,7 +1163,8 @@ struct Refiner {
     NvtxRange nvtx("gqm:flip_flop");
     count_launch(1);
     return gqm_flip_loop_launch(&M, sizeof(M), &fl, sizeof(fl), bars, &ds->team, pred_mode,
-                                loop_blocks[tune.check_minb], tune.check_minb, tune.small_limit, tune.small_cluster,
+                                std::max(1, loop_blocks[tune.check_minb] / sharers), tune.check_minb, tune.small_limit,
+                                tune.small_cluster,
                                 ktm, stm, st);
   }
   // Blocks that a refinement uses.  A barrier of several blocks costs several
@@ -1174,7 +1176,7 @@ struct Refiner {
   // and 148 (steps of up to 512 triangles by the first block).
   int team_blocks(int nt) const {
     if (nt <= 2048) return 1;
-    const int most = std::min(tune.step_grid, loop_blocks[tune.check_minb]);
+    const int most = std::min(tune.step_grid, std::max(1, loop_blocks[tune.check_minb] / sharers));
     return std::max(1, std::min(most, std::max(16, nt / 512)));
   }
 
@@ -2224,7 +2226,12 @@ int gqm_refine_batch(int ndomains, const gqm_cdt_in *in, gqm_cdt_out *out, const
       if (k >= ndomains || first_err.load() != 0) break;
       int d = order[k];
       int rc = GQM_OK;
-      if (!ctx) rc = gqm_context_create(opt[d].device, &ctx);
+      if (!ctx) {
+        rc = gqm_context_create(opt[d].device, &ctx);
+        // launches that all fit run side by side; each on the whole GPU would
+        // run one after another
+        if (rc == GQM_OK) ctx->r.sharers = workers;
+      }
       gqm_stats st;
       if (rc == GQM_OK) rc = gqm_context_run(ctx, &in[d], 0, &opt[d], &st);
       if (rc == GQM_OK) rc = gqm_context_result(ctx, &out[d]);
