@@ -31,6 +31,7 @@
 #define GQM_GTID ((int)(gqm_team_rank * blockDim.x + threadIdx.x))
 #define GQM_GSIZE ((int)(gqm_team_blocks * blockDim.x))
 #define GQM_BLOCK0 (gqm_team_rank == 0)
+#define GQM_WALK_CALL __noinline__
 #elif defined(GQM_CLUSTER_MODE)
 #define GQM_KERNEL __device__
 #define GQM_WALK_BOUNDS
@@ -38,6 +39,7 @@
 #define GQM_GTID ((int)(blockIdx.x * blockDim.x + threadIdx.x))
 #define GQM_GSIZE ((int)(gridDim.x * blockDim.x))
 #define GQM_BLOCK0 (blockIdx.x == 0)
+#define GQM_WALK_CALL
 #else
 #define GQM_KERNEL __global__
 #define GQM_WALK_BOUNDS __launch_bounds__(256, GQM_WALK_MIN_BLOCKS)
@@ -45,6 +47,7 @@
 #define GQM_GTID ((int)(blockIdx.x * blockDim.x + threadIdx.x))
 #define GQM_GSIZE ((int)(gridDim.x * blockDim.x))
 #define GQM_BLOCK0 (blockIdx.x == 0)
+#define GQM_WALK_CALL
 #endif
 
 namespace gqm {
@@ -1683,7 +1686,7 @@ GQM_KERNEL void k_remove_losers(Mesh M, const int *bad, const int *dn, const int
 // the same edges as one that tests each neighbour when it gets to it.
 __device__ __forceinline__ unsigned cavity_hash(int t) { return ((unsigned)t * 2654435761u) >> 26; }
 template <int PRED>
-__device__ int cavity_walk(const Mesh &M, int gen, int sink, int direction, double2 cc, int badIndex, int *out,
+__device__ GQM_WALK_CALL int cavity_walk(const Mesh &M, int gen, int sink, int direction, double2 cc, int badIndex, int *out,
                            int stride) {
   int region[kCavityCap], loop[kCavityCap];  // loop: (triangle << 2) | edge to resume at
   uint8_t inside[kCavityCap];                // per frame: neighbours whose circumcircle holds cc
@@ -1762,6 +1765,74 @@ __device__ int cavity_walk(const Mesh &M, int gen, int sink, int direction, doub
   return 0;
 }
 
+#if defined(GQM_CTA_MODE) && !defined(GQM_HOST_EMU)
+// The same cavity by sixteen lanes: the triangles found so far are a list
+// spread over the lanes' registers, and every pass tests the next sixteen of
+// their edges together, each with its own loads (link and subsegment, then the
+// neighbour's row, then its points).  Which triangles the cavity holds does not
+// depend on the order in which they are reached, so a cavity within the cap is
+// claimed when it is complete; of a larger one the reference claims the first
+// fifty in its own order, and that one is left to cavity_walk (-1 is returned,
+// nothing is claimed).
+//
+// Bound by latency: the walk waits three dependent loads for every triangle, a
+// pass here for every step outward from the sink.  Outside its flip loops a
+// refinement of 3,000 points takes 4.2 ms instead of 5.5 ms, one of 10,000
+// points 3.6 ms instead of 4.0 ms, one of 100,000 points 6.9 ms instead of 7.1 ms.
+template <int PRED>
+__device__ __forceinline__ int cavity_group(const Mesh &M, int gen, int sink, int direction, double2 cc, int badIndex,
+                                            int *out, int stride) {
+  const int lane = (int)(threadIdx.x & 31u), gl = lane & 15;
+  const unsigned gm = 0xffffu << (lane & 16);
+  static_assert(kCavityCap <= 64, "four entries a lane");
+  int r0 = gl == 0 ? sink : -1, r1 = -1, r2 = -1, r3 = -1;  // entries gl, gl + 16, gl + 32, gl + 48
+  int size = 1;
+  for (int head = 0; head < 3 * size;) {
+    const int p = head + gl, end = 3 * size;
+    const bool has = p < end;
+    const int idx = has ? p / 3 : 0, e = p - 3 * (p / 3), own = (lane & 16) | (idx & 15);
+    const int t0 = __shfl_sync(gm, r0, own), t1 = __shfl_sync(gm, r1, own), t2 = __shfl_sync(gm, r2, own),
+              t3 = __shfl_sync(gm, r3, own);
+    const int t = idx < 16 ? t0 : idx < 32 ? t1 : idx < 48 ? t2 : t3;
+    int found = -1;
+    if (has) {
+      const int link = ld1(M.tn, t, e), sg = ld1(M.tsg, t, e);
+      if (link != -1 && (sg == -1 || (t == sink && e == direction))) {
+        const int4 q = M.tv[dtri(link)];
+        if (incircle<PRED>(M.pts[q.x], M.pts[q.y], M.pts[q.z], cc) > 0) found = dtri(link);
+      }
+    }
+    head = min(head + 16, end);
+    unsigned in = __ballot_sync(gm, found >= 0) & gm;
+    while (in) {
+      const int c = __shfl_sync(gm, found, __ffs(in) - 1);
+      in &= in - 1;
+      if (__any_sync(gm, r0 == c || r1 == c || r2 == c || r3 == c)) continue;
+      if (size == kCavityCap) return -1;
+      if (gl == (size & 15)) {
+        if (size < 16)
+          r0 = c;
+        else if (size < 32)
+          r1 = c;
+        else if (size < 48)
+          r2 = c;
+        else
+          r3 = c;
+      }
+      ++size;
+    }
+  }
+  const int r[4] = {r0, r1, r2, r3};
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (16 * k + gl < size) {
+      claim(M, gen, r[k], badIndex);
+      out[(long)(16 * k + gl) * stride] = r[k];
+    }
+  return size;
+}
+#endif
+
 // kernelMarkCavities: claim every cavity triangle (atomicMin of the bad index);
 // an oversized cavity makes its candidate an unconditional winner (negated
 // index).  cavn[k] = stored cavity size (0 for an oversized one).
@@ -1770,10 +1841,30 @@ GQM_KERNEL void GQM_WALK_BOUNDS k_cavity_mark(Mesh M, const int *dn, const int *
                               int *ilist, int *cav, int *cavn, int stride, FlipLists L) {
   int n = *dn;
   const int gen = L.c->gen - kGenCavity;
+#if defined(GQM_CTA_MODE) && !defined(GQM_HOST_EMU)
+  // Sixteen lanes a candidate while the team needs at most eight passes for
+  // them; the grid kernel's inputs have more candidates than that in most rounds
+  // (with both ways in it, its walk took 25 ms of a refinement of 2,000,000
+  // points outside the flip loops instead of 23 ms).
+  if (2 * n <= GQM_GSIZE) {
+    const int gl = (int)(threadIdx.x & 15u);
+    for (int k = GQM_GTID >> 4; k < n; k += GQM_GSIZE >> 4) {
+      if (imark[k] < 0) continue;
+      const int badIndex = ilist[k], sk = sinks[k];
+      int c = cavity_group<PRED>(M, gen, sk >> 2, sk & 3, center[k], badIndex, cav + k, stride);
+      __syncwarp(0xffffu << (threadIdx.x & 16u));  // every lane has read ilist[k]
+      if (gl) continue;
+      if (c < 0) c = cavity_walk<PRED>(M, gen, sk >> 2, sk & 3, center[k], badIndex, cav + k, stride);
+      if (c < 0) ilist[k] = negate_idx(badIndex);
+      cavn[k] = c < 0 ? 0 : c;
+    }
+    return;
+  }
+#endif
   GS_LOOP(k, n) {
     if (imark[k] < 0) continue;
-    int badIndex = ilist[k];
-    int c = cavity_walk<PRED>(M, gen, sinks[k] >> 2, sinks[k] & 3, center[k], badIndex, cav + k, stride);
+    const int badIndex = ilist[k];
+    const int c = cavity_walk<PRED>(M, gen, sinks[k] >> 2, sinks[k] & 3, center[k], badIndex, cav + k, stride);
     if (c < 0) ilist[k] = negate_idx(badIndex);
     cavn[k] = c < 0 ? 0 : c;
   }

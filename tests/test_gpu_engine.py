@@ -55,3 +55,18 @@ def test_batch_teams_match_oracle(gpu, sizes):
             want, info = oracle_py.refine(d, 20.0, 1, 1)
             _same(g, want)
             assert st["rounds"] == info["rounds"]
+
+
+@pytest.mark.parametrize("ring", [30, 52, 53, 120, 700])
+def test_large_cavities_match_oracle(gpu, ring):
+    """Points on a circle: the first Steiner points' cavities hold nearly every
+    triangle, on both sides of the cap of fifty."""
+    a = 2 * np.pi * (np.arange(ring) + 0.3 * np.random.default_rng(ring).uniform(-1, 1, ring)) / ring
+    pts = np.stack([100 * np.cos(a), 100 * np.sin(a)], 1)
+    cdt = inputs.build_cdt(pts, np.zeros((0, 2), np.int32))
+    got, st = refine.refine(cdt, 20.0)
+    want, info = oracle_py.refine(cdt, 20.0, 1, 1)
+    _same(got, want)
+    assert st["rounds"] == info["rounds"]
+    one, _ = refine.refine_batch_persistent([cdt], 20.0)
+    _same(one[0], want)
