@@ -25,13 +25,23 @@ struct HostCopy {
   size_t bytes;
 };
 
+// Threads that a copy of `bytes` in `pieces` pieces is worth, the calling one
+// included: one for every megabyte.  Starting a thread costs as much as copying
+// a few hundred kilobytes, and a small result's six arrays had one each.
+static inline int host_copy_threads(size_t bytes, size_t pieces) {
+  const size_t most = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
+  return (int)std::max<size_t>(1, std::min({pieces, most, bytes >> 20}));
+}
+
 static inline void host_copy(std::initializer_list<HostCopy> list) {
   constexpr size_t kPiece = 8u << 20;
   std::vector<HostCopy> pieces;
   for (const HostCopy &c : list)
     for (size_t o = 0; o < c.bytes; o += kPiece)
       pieces.push_back({(char *)c.dst + o, (const char *)c.src + o, std::min(kPiece, c.bytes - o)});
-  int nt = (int)std::min<size_t>(pieces.size(), std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
+  size_t bytes = 0;
+  for (const HostCopy &c : list) bytes += c.bytes;
+  const int nt = host_copy_threads(bytes, pieces.size());
   if (nt <= 1) {
     for (const HostCopy &c : pieces) memcpy(c.dst, c.src, c.bytes);
     return;
@@ -69,7 +79,9 @@ static inline void host_copy_streamed(const List &list, char *dst_base, size_t s
       done[k].store(1, std::memory_order_release);
     }
   };
-  const int nt = (int)std::min<size_t>(np, std::max(1u, std::min(16u, std::thread::hardware_concurrency())));
+  size_t bytes = 0;
+  for (const HostCopy &c : list) bytes += c.bytes;
+  const int nt = host_copy_threads(bytes, np);
   std::vector<std::thread> pool;
   for (int t = 1; t < nt; ++t) pool.emplace_back(work);
   // the calling thread hands on the completed front, and copies when it has nothing to hand on
