@@ -47,22 +47,15 @@ sys.path.insert(0, ROOT)
 
 METRIC = "output triangles/s at theta=20 deg, 1 B200 (learned vs plain); output vertex count"
 
-# Algorithmic bytes of the flip-step check kernel (k_check_flip2, the
+# Algorithmic bytes of the check phase of a flip step (flip_check, the
 # kernelCheckFlipping of GPU_Refine/refine.cu:778-1070) per active triangle:
 # the list entry (4), the triangle's vertices, neighbours and subsegments
 # (3 x 12), the redundant flags of its vertices (3), its three points (48),
 # per edge the neighbour's flip flag, opposite vertex, its flag and point
 # (3 x 22), and the deferred-clear byte written back (1).
 CHECK_BYTES_PER_ITEM = 4 + 36 + 3 + 48 + 66 + 1
-# DRAM bytes (read + write) per active triangle of the same kernel, from
-# `ncu --set full` on its first launch of the 1,000,000-point clustered case
-# (profiles/k_check_flip2_clustered1M.md: 72.22 MB for 162,684 triangles).
-CHECK_DRAM_BYTES_PER_ITEM = 72.22e6 / 162684
-# FP64-pipe utilisation of the same launch (sm__inst_executed_pipe_fp64, % of
-# peak sustained active): the exact-predicate filters are a small part of its work.
-CHECK_FP64_PIPE_PCT = 4.26
-# Algorithmic bytes of one whole flip step, for the small-step kernel (it runs
-# every phase of a step in one launch), per active triangle: the check
+# Algorithmic bytes of one whole flip step, for the small steps (one block runs
+# every phase of them), per queued triangle: the check
 # (CHECK_BYTES_PER_ITEM), the winner test (list entry 4, deferred-clear byte
 # 1, flip orientation 1, the claim words of the triangle and its partner 8)
 # and the filter into the next active set (queue entry 4, flip flag 1, status
@@ -442,11 +435,11 @@ def run_reference(args, rank, world):
 
 
 def kernel_rooflines(probe, ms_step, peak, peak_kind):
-    """Roofline entries of the two kernels that take most of the device time,
-    from the per-launch device timers of one probed refinement: the grid-wide
-    flip-step check kernel (CHECK_BYTES_PER_ITEM per active triangle) and the
-    small-step kernel (STEP_BYTES_PER_ITEM per active triangle plus
-    STEP_BYTES_PER_WINNER per flip applied, summed over the steps it ran)."""
+    """Roofline entries of the two parts of the flip-flop loops' launch that take
+    most of the device time, from the device timers of one probed refinement: the
+    check phase of the steps run by all blocks (CHECK_BYTES_PER_ITEM per active
+    triangle) and the small steps (STEP_BYTES_PER_ITEM per queued triangle plus
+    STEP_BYTES_PER_WINNER per flip applied)."""
     out = []
     launches = max(int(probe["check_launches"]), 1)
     if probe["check_ms"] > 0:
@@ -454,13 +447,11 @@ def kernel_rooflines(probe, ms_step, peak, peak_kind):
         launch_s = probe["check_ms"] / 1e3 / launches
         ach = CHECK_BYTES_PER_ITEM * items / launch_s / 1e9
         out.append({"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
-                    "traffic": CHECK_DRAM_BYTES_PER_ITEM * items, "peak_kind": peak_kind,
-                    "kernel": "k_check_flip2 (grid-wide flip-step check)", "bytes_per_item": CHECK_BYTES_PER_ITEM,
+                    "traffic": None, "peak_kind": peak_kind,
+                    "kernel": "k_flip_loop, check phase of the steps run by all blocks",
+                    "bytes_per_item": CHECK_BYTES_PER_ITEM,
                     "launches": launches, "items_per_launch": items, "avg_launch_us": launch_s * 1e6,
-                    "share_of_step": probe["check_ms"] / ms_step,
-                    "traffic_note": "ncu DRAM bytes per active triangle of the 1M-point capture "
-                                    "(profiles/k_check_flip2_clustered1M.md) times this launch's items",
-                    "fp64_pipe_pct_ncu": CHECK_FP64_PIPE_PCT})
+                    "share_of_step": probe["check_ms"] / ms_step})
     sl = max(int(probe["small_launches"]), 1)
     if probe["small_ms"] > 0:
         alg = STEP_BYTES_PER_ITEM * probe["small_items"] + STEP_BYTES_PER_WINNER * probe["small_winners"]
@@ -468,7 +459,7 @@ def kernel_rooflines(probe, ms_step, peak, peak_kind):
         ach = alg / sl / launch_s / 1e9
         out.append({"bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak,
                     "traffic": None, "peak_kind": peak_kind,
-                    "kernel": "small-step kernel (whole flip steps of small active sets in one launch)",
+                    "kernel": "k_flip_loop, small steps (whole flip steps by one block)",
                     "bytes_per_item": STEP_BYTES_PER_ITEM, "bytes_per_winner": STEP_BYTES_PER_WINNER,
                     "launches": sl, "items_per_launch": probe["small_items"] / sl,
                     "winners_per_launch": probe["small_winners"] / sl, "avg_launch_us": launch_s * 1e6,

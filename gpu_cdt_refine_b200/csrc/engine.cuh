@@ -44,7 +44,6 @@ struct EngineRun {
   MlpDev mlp;
   double theta, max_area;
   long long max_rounds;
-  int fresh;  // buffers carry nothing from earlier runs (stamps, claims and tags are cleared)
   // results
   int status, need_grow, out_np, out_nt, out_ns, rounds;
   int last_point, last_triangle;

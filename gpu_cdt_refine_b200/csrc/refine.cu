@@ -263,7 +263,6 @@ struct PPtLive {
   __device__ bool operator()(int i) const { return !(ps[i] & PS_DELETED); }
 };
 
-__global__ void k_fill(int *a, int n, int v) { GS_LOOP(i, n) a[i] = v; }
 __global__ void k_copy(int *dst, const int *src, const int *dn) {
   int n = *dn;
   GS_LOOP(i, n) dst[i] = src[i];

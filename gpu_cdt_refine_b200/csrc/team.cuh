@@ -21,9 +21,9 @@ struct BlockTeam {
 };
 
 // `nb` blocks, all of them resident (a cooperative launch).  A barrier adds one
-// arrival per block to a word that only grows; a block
-// waits until all arrivals of its own barrier have been counted.  The arrival
-// is a reduction with no answer to wait for, and the wait polls one word.
+// arrival per block to a word that only grows; a block waits until all arrivals
+// of its own barrier have been counted.  The arrival is a reduction with no
+// answer to wait for, and the wait polls one word.
 struct GridBar {
   unsigned long long arrived;  // arrivals of all barriers
   unsigned long long base;     // arrivals when the current launch began
