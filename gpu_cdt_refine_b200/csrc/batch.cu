@@ -507,7 +507,7 @@ int run_batch(DevCache &C, const std::vector<int> &ids, const gqm_cdt_in *in, gq
   grid = std::min<long>(grid, (long)((have - fixed) / arena));
 #else
   (void)mem_fraction;
-  grid = 1;
+  grid = std::min(grid, std::max(1L, (long)GQM_EMU_BLOCKS / nb));
 #endif
   if (grid < 1) return GQM_ERR_MEMORY;
   if (grow_dev(&C.d_in, &C.in_cap, in_bytes) || grow_dev(&C.d_out, &C.out_cap, out_bound) ||
@@ -620,7 +620,8 @@ int run_batch(DevCache &C, const std::vector<int> &ids, const gqm_cdt_in *in, gq
   cudaEventRecord(C.e0, C.st);
   TeamState *teams = reinterpret_cast<TeamState *>(C.d_teams);
 #ifdef GQM_HOST_EMU
-  V.fn(C.d_jobs, C.d_order, n, C.d_next, C.d_arena, arena, teams, 1, jobs[0].pred);
+  GQM_EMU_GRID((int)grid * nb,
+               V.fn(C.d_jobs, C.d_order, n, C.d_next, C.d_arena, arena, teams, nb, jobs[0].pred));
 #else
   {
     cudaLaunchConfig_t cfg = {};
@@ -754,6 +755,8 @@ int setup_dev(DevCache &C, int device) {
     return GQM_ERR_MEMORY;
 #ifndef GQM_HOST_EMU
   cudaDeviceGetAttribute(&C.sms, cudaDevAttrMultiProcessorCount, device);
+#else
+  C.sms = GQM_EMU_BLOCKS;
 #endif
   C.init = true;
   return GQM_OK;
@@ -855,10 +858,7 @@ int gqm_refine_one_launch(const void *scratch, size_t scratch_bytes, const void 
 #ifdef GQM_HOST_EMU
   (void)blocks;
   (void)st;
-  if (pred)
-    k_refine_one<1>(S, c, r, ts, small_limit, kt, stm);
-  else
-    k_refine_one<0>(S, c, r, ts, small_limit, kt, stm);
+  GQM_EMU_GRID(blocks, (pred ? k_refine_one<1> : k_refine_one<0>)(S, c, r, ts, small_limit, kt, stm));
   return GQM_OK;
 #else
   cudaLaunchConfig_t cfg = {};

@@ -152,10 +152,15 @@ struct Engine {
   template <class F, class Mp>
   __device__ __noinline__ int compact(F f, Mp m, int lo, int hi, int *out, int *count) {
 #ifdef GQM_HOST_EMU
-    int k = 0;
-    for (int i = lo; i < hi; ++i)
-      if (f(i)) out[k++] = m(i);
-    *count = k;
+    int *part = ts.part[parity];
+    parity ^= 1;
+    if (T.rank == 0) {
+      part[0] = 0;
+      for (int i = lo; i < hi; ++i)
+        if (f(i)) out[part[0]++] = m(i);
+    }
+    TSYNC();
+    *count = part[0];
     return GQM_OK;
 #else
     constexpr int kItems = 16;

@@ -65,7 +65,7 @@ size_t gqm_flip_bar_bytes() { return 2 * sizeof(gqm::GridBar); }
 int gqm_flip_max_blocks(int budget) {
 #ifdef GQM_HOST_EMU
   (void)budget;
-  return 1;
+  return GQM_EMU_BLOCKS;
 #else
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -98,7 +98,7 @@ int gqm_flip_loop_launch(const void *mesh, size_t mesh_bytes, const void *lists,
 #ifdef GQM_HOST_EMU
   (void)blocks;
   (void)st;
-  gqm::loop_fn(pred, budget)(M, L, b, team, small_limit, small_team, kt, stm);
+  GQM_EMU_GRID(blocks, gqm::loop_fn(pred, budget)(M, L, b, team, small_limit, small_team, kt, stm));
   return GQM_OK;
 #else
   cudaLaunchConfig_t cfg = {};

@@ -366,15 +366,21 @@ struct FlipCnt {
   int nred[2];   // triangles whose claim may name a redundant point
   int nlate[2];  // subseg2tri stores that another winner competes with
 };
+// What a run of small steps leaves for the team's other blocks.
+struct FlipOut {
+  FlipCnt cnt;
+  int gen, steps, status;  // status: how the run ended (FLIP_*)
+  unsigned epoch;
+};
 struct FlipCtl {
   int gen;         // generation of the pushes between loops (stamps, claims)
   unsigned epoch;  // launch epoch of the subseg2tri stores (all kernels share it)
   FlipCnt cnt;
+  FlipOut out[2];  // by turns, see flip_loop
   int steps;        // flip steps executed (all loops)
   int small_steps;  // of which steps run by the small-step team
   int cap_hit;      // the step bound stopped a loop
   int ran;          // loops run since the reset
-  int small_status; // how the last run of small steps ended (FLIP_*)
   long long cap;    // bound on the steps of one loop
   int *errp;        // device error word (GQM_ERR_ROUND_LIMIT on cap_hit)
   // device time of the loops (%globaltimer from loop entry to loop end)
@@ -815,8 +821,7 @@ __device__ __noinline__ void flip_check(const Mesh &M, const int *q, int n, int 
     for (long i = tid; i < words; i += size) L.wbits[i] = 0u;
   }
 #ifdef GQM_HOST_EMU
-  (void)size;
-  for (int k = tid; k < n; ++k) {
+  for (int k = tid; k < n; k += size) {
     const int index = q[k];
     const int4 p = M.tv[index], nb = M.tn[index], sg = M.tsg[index];
     int4 r = make_int4(index, FD_DEAD, -1, 0);
@@ -1085,8 +1090,7 @@ __device__ __forceinline__ void fix_edge(const Mesh &M, const FlipQ &Q, uint32_t
 __device__ __noinline__ void flip_fix(const Mesh &M, int n, const FlipQ &Q, uint32_t epoch, const FlipLists &L,
                                       const int4 *rec, int *nlate, int tid, int size) {
 #ifdef GQM_HOST_EMU
-  (void)size;
-  for (int k = tid; k < n; ++k)
+  for (int k = tid; k < n; k += size)
     if (rec[k].y >= 0 && (rec[k].y & FD_WON))
       for (int j = 0; j < 4; ++j) fix_edge(M, Q, epoch, L, rec[k], j, nlate);
 #else
@@ -1234,29 +1238,35 @@ __device__ __forceinline__ bool flip_loop(const Mesh &M, const FlipLists &L, Sma
                                           GridTeam *S, KTimer *ktm, KTimer *stm) {
   FlipCtl *c = L.c;
   FlipRegs R{vload(&c->gen), (unsigned)vload((const int *)&c->epoch), vload(&c->steps)};
+  FlipCnt *cnt = &c->cnt;
   const int entry = R.steps;
   const int timed = ktm ? ktm->on : 0;
   const int small_blocks = S ? S->nb : 1;
   const unsigned long long t0 = G.lead() ? global_ns() : 0;
-  int status = FLIP_GO;
-  // Every block takes the same way through the loop: what it decides on (list
-  // lengths, the control block) was written before the last barrier of all
-  // blocks and is not written again before the next.
+  int status = FLIP_GO, turn = 0;
+  // Every block takes the same way through the loop: the words it decides on
+  // were complete before the last barrier of all blocks (before the launch, at
+  // the loop's entry) and stay as they are until the next.  A run of small steps
+  // therefore works on a copy of the list lengths and leaves what it comes to
+  // in c->out[turn], which the others read behind that barrier; the one it left
+  // before is not read any more by then.
   while (status == FLIP_GO) {
-    const int n = vload(&c->cnt.qn[R.gen & 1]);
+    const int n = vload(&cnt->qn[R.gen & 1]);
     if (n == 0) break;
     if (n > small_limit) {
-      status = flip_step<PRED>(M, L, &c->cnt, R, entry, G, (R.gen & 1) ? L.q1 : L.q0, n, L.rec, timed ? ktm : nullptr,
+      status = flip_step<PRED>(M, L, cnt, R, entry, G, (R.gen & 1) ? L.q1 : L.q0, n, L.rec, timed ? ktm : nullptr,
                                nullptr);
       continue;
     }
-    const int steps0 = R.steps;
+    FlipOut *o = &c->out[turn];
+    turn ^= 1;
     if (G.rank < small_blocks) {
       const unsigned long long s0 = timed && G.lead() ? global_ns() : 0;
+      const int steps0 = R.steps;
       int items = 0, wins = 0, m = n;
       if (!S) {
         BlockTeam B;
-        if (B.lead()) sh.cnt = c->cnt;
+        if (B.lead()) sh.cnt = *cnt;
         B.sync();
         while (status == FLIP_GO && m > 0 && m <= small_limit) {
           items += m;
@@ -1264,30 +1274,32 @@ __device__ __forceinline__ bool flip_loop(const Mesh &M, const FlipLists &L, Sma
                                    m <= kSmallCap ? sh.rec : L.rec, nullptr, timed ? &wins : nullptr);
           m = vload(&sh.cnt.qn[R.gen & 1]);
         }
-        B.sync();
-        if (B.lead()) c->cnt = sh.cnt;
+        if (B.lead()) o->cnt = sh.cnt;
       } else {
+        if (S->lead()) o->cnt = *cnt;
+        if (!S->sync()) status = FLIP_BROKEN;
         while (status == FLIP_GO && m > 0 && m <= small_limit) {
           items += m;
-          status = flip_step<PRED>(M, L, &c->cnt, R, entry, *S, (R.gen & 1) ? L.q1 : L.q0, m, L.rec, nullptr,
+          status = flip_step<PRED>(M, L, &o->cnt, R, entry, *S, (R.gen & 1) ? L.q1 : L.q0, m, L.rec, nullptr,
                                    timed ? &wins : nullptr);
-          m = vload(&c->cnt.qn[R.gen & 1]);
+          m = vload(&o->cnt.qn[R.gen & 1]);
         }
       }
       if (G.lead()) {
-        c->gen = R.gen;
-        c->epoch = R.epoch;
-        c->steps = R.steps;
+        o->gen = R.gen;
+        o->epoch = R.epoch;
+        o->steps = R.steps;
+        o->status = status;
         c->small_steps += R.steps - steps0;
-        c->small_status = status;
         if (timed) ktimer_add(stm, s0, items, wins);
       }
     }
     if (!G.sync()) return false;
-    R.gen = vload(&c->gen);
-    R.epoch = (unsigned)vload((const int *)&c->epoch);
-    R.steps = vload(&c->steps);
-    status = vload(&c->small_status);
+    cnt = &o->cnt;
+    R.gen = vload(&o->gen);
+    R.epoch = (unsigned)vload((const int *)&o->epoch);
+    R.steps = vload(&o->steps);
+    status = vload(&o->status);
   }
   if (status == FLIP_BROKEN || !G.sync()) return false;  // nobody reads the control block any more
   if (G.lead()) {
@@ -2196,7 +2208,7 @@ GQM_KERNEL void k_emit_pstatus(Mesh M, int np, uint8_t *pstat) {
 GQM_KERNEL void k_learned_place(Mesh M, const int *bad, const int *dn, MlpDev P, double2 *center,
                                 unsigned long long *ctr) {
 #ifdef GQM_HOST_EMU
-  const int n = *dn;
+  const int n = GQM_BID == 0 ? *dn : 0;
   for (int k = 0; k < n; ++k) {
     const int t = bad[k];
     const int4 v = M.tv[t];

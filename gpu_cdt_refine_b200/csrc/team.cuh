@@ -5,6 +5,15 @@
 
 #include "../../include/gqm_refine.h"
 
+// A host build of the kernels runs one block of one thread, unless it defines
+// these: the blocks of a launch, the launch of so many, and a block's wait for
+// a word to reach a value (false: it never will).
+#if defined(GQM_HOST_EMU) && !defined(GQM_EMU_BLOCKS)
+#define GQM_EMU_BLOCKS 1
+#define GQM_EMU_GRID(blocks, call) call
+#define GQM_EMU_WAIT(word, target) true
+#endif
+
 namespace gqm {
 
 __device__ __forceinline__ int vload(const int *p) { return *(const volatile int *)p; }
@@ -41,7 +50,13 @@ struct GridTeam {
   __device__ __forceinline__ bool lead() const { return rank == 0 && threadIdx.x == 0; }
   __device__ __forceinline__ bool sync() {
 #ifdef GQM_HOST_EMU
-    return true;
+    if (nb == 1) return true;
+    target += (unsigned long long)nb;
+    ++bar->arrived;
+    if (GQM_EMU_WAIT(&bar->arrived, target)) return true;
+    bar->broken = 1;
+    if (*err == 0) *err = code;
+    return false;
 #else
     if (nb == 1) {
       __syncthreads();

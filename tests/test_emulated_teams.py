@@ -1,0 +1,56 @@
+"""The cooperative launches (csrc/team.cuh) as several blocks on the CPU: the
+refiner's own sources compiled with tests/emu/team_emu.h, whose blocks run one
+at a time from barrier to barrier in a chosen order.  Whatever the order, every
+block has to take the same way through the barriers and the mesh is the
+oracle's byte for byte.  Order 0 lets the first block run ahead of all others
+(it runs the small flip steps), order 1 lets it come last."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from gpu_cdt_refine_b200 import inputs, refine
+from oracle import oracle_py
+
+from test_emulated_kernels import _same, emulated  # noqa: F401  (fixture)
+
+teams = pytest.mark.parametrize("emulated", ["libgqm_emu_teams.so"], indirect=True)
+
+
+def _schedule(order):
+    L = refine.lib()
+    L.gqm_emu_schedule.argtypes = [ctypes.c_int]
+    L.gqm_emu_schedule(order)
+    return L
+
+
+@teams
+@pytest.mark.parametrize("order", [0, 1, 2, 3])
+@pytest.mark.parametrize("points", [1500, 3000])  # one launch; the flip loop's own launch
+@pytest.mark.parametrize("shape", [dict(), dict(small_limit=-1), dict(small_limit=40), dict(small_cluster=8)],
+                         ids=["default", "no small steps", "both", "small team"])
+def test_flip_loop_in_any_order_of_blocks(emulated, order, points, shape):  # noqa: F811
+    cdt = inputs.plain_small(seed=7100 + points, n=points, nseg=points // 15)
+    L = _schedule(order)
+    ctx = refine.Context(0)
+    try:
+        ctx.set_tuning(**shape)
+        st = ctx.run_host(cdt, refine.make_options(20.0, 1, 1))
+        got = ctx.result()
+    finally:
+        ctx.close()
+    assert L.gqm_emu_stuck_count() == 0
+    want, info = oracle_py.refine(cdt, 20.0, 1, 1)
+    _same(got, want)
+    assert st["rounds"] == info["rounds"] and st["flip_steps"] > 0
+
+
+@teams
+@pytest.mark.parametrize("order", [0, 1, 2])
+def test_batch_teams_in_any_order_of_blocks(emulated, order):  # noqa: F811
+    doms = [inputs.plain_small(seed=7200 + i, n=n, nseg=n // 15) for i, n in enumerate([900, 300])]
+    L = _schedule(order)
+    got, _ = refine.refine_batch_persistent(doms, 20.0)
+    assert L.gqm_emu_stuck_count() == 0
+    for d, g in zip(doms, got):
+        _same(g, oracle_py.refine(d, 20.0, 1, 1)[0])
