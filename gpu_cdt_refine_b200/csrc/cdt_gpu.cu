@@ -135,10 +135,11 @@ CDEV unsigned fbits(float f) {
 }
 
 // Counters in ctr[].  kNd and kNc hold two each (dirty list and candidates of
-// alternating flip rounds); from kStop on: the launch of the insertion rounds.
+// alternating flip rounds); from kStop on: the launch of the insertion rounds;
+// kOut: two sets of eight words (see lawson).
 enum {
   kErr = 0, kNtri, kNpend, kNd, kNc = kNd + 2, kFlips = kNc + 2, kTot, kMiss, kHcnt, kRecFlips,
-  kStop, kInsRounds, kFlipRounds, kStamp, kTag, kParity, kNctr = 24
+  kStop, kInsRounds, kFlipRounds, kStamp, kTag, kOut = 24, kNctr = kOut + 16
 };
 struct Dm {
   const double2 *P;
@@ -680,57 +681,73 @@ struct FlipRegs {  // registers of every thread
   int stamp, tag, p, rounds;
 };
 // One flip round over the n dirty triangles of list R.p by a team: check, win
-// and apply, a barrier behind each.
+// and apply, a barrier behind each.  cnt: the lengths of the two dirty lists and
+// of the two candidate lists (the words at ctr[kNd], or a copy).
 template <class Team>
-CDEV bool flip_round(const Dm &M, const Lists &L, Team &T, FlipRegs &R, int n) {
+CDEV bool flip_round(const Dm &M, const Lists &L, int *cnt, Team &T, FlipRegs &R, int n) {
   ++R.stamp;
   const int t2 = ++R.tag, p = R.p, q = p ^ 1;
-  if (T.lead()) L.ctr[kNd + q] = 0;
-  flip_check(M, p ? L.D2 : L.D, n, t2 - 1, R.stamp, L.C, L.ctr + kNc + p, T.tid(), T.size());
+  if (T.lead()) cnt[q] = 0;
+  flip_check(M, p ? L.D2 : L.D, n, t2 - 1, R.stamp, L.C, cnt + 2 + p, T.tid(), T.size());
   if (!T.sync()) return false;
-  const int nc = vload(L.ctr + kNc + p);
+  const int nc = vload(cnt + 2 + p);
   R.p = q;
   R.rounds++;
   if (nc == 0) return true;  // nothing illegal: the next list is empty
-  if (T.lead()) L.ctr[kNc + q] = 0;
+  if (T.lead()) cnt[2 + q] = 0;
   flip_win(M, L.C, nc, R.stamp, L.wf, T.tid(), T.size());
   if (!T.sync()) return false;
-  flip_apply(M, L.C, nc, L.wf, R.stamp, t2, q ? L.D2 : L.D, L.ctr + kNd + q, L.ctr + kFlips, T.tid(), T.size());
+  flip_apply(M, L.C, nc, L.wf, R.stamp, t2, q ? L.D2 : L.D, cnt + q, L.ctr + kFlips, T.tid(), T.size());
   return T.sync();
 }
 // Lawson flips over the dirty list D (count in ctr[kNd], tag R.tag) until no
-// edge is illegal.
+// edge is illegal.  Every block takes the same way through the loop: the words
+// it decides on were complete before the last barrier of all blocks (before the
+// launch, at a launch's start) and stay as they are until the next.  The first
+// block's small rounds therefore count in a copy of the lengths and leave what
+// they come to in a set of words of their own, one of two by turns, which the
+// others read behind that barrier.
 __device__ __noinline__ bool lawson(const Dm &M, const Lists &L, GridTeam &T, FlipRegs &R) {
+  __shared__ int small[4];
+  int *cnt = L.ctr + kNd;
+  const int entry = R.rounds;
   R.p = 0;
-  for (int guard = 0;; ++guard) {
-    const int n = vload(L.ctr + kNd + R.p);
+  for (int turn = 0;;) {
+    const int n = vload(cnt + R.p);
     if (n == 0) return true;
-    if (guard > (1 << 24)) {
+    if (R.rounds - entry > (1 << 24)) {
       if (T.lead()) set_err(M.err, GQM_CDT_ERR_INTERNAL);
       return true;
     }
     if (n > kSmallDirty || T.nb == 1) {
-      if (!flip_round(M, L, T, R, n)) return false;
+      if (!flip_round(M, L, cnt, T, R, n)) return false;
       continue;
     }
+    int *out = L.ctr + kOut + 8 * turn;
+    turn ^= 1;
     if (T.rank == 0) {
       BlockTeam B;
-      for (int m = n; m > 0 && m <= kSmallDirty && guard <= (1 << 24); ++guard) {
-        flip_round(M, L, B, R, m);
-        m = vload(L.ctr + kNd + R.p);
+      if (threadIdx.x == 0)
+        for (int i = 0; i < 4; ++i) small[i] = cnt[i];
+      B.sync();
+      for (int m = n; m > 0 && m <= kSmallDirty && R.rounds - entry <= (1 << 24);) {
+        flip_round(M, L, small, B, R, m);
+        m = vload(small + R.p);
       }
       if (T.lead()) {
-        L.ctr[kStamp] = R.stamp;
-        L.ctr[kTag] = R.tag;
-        L.ctr[kParity] = R.p;
-        L.ctr[kFlipRounds] = R.rounds;
+        for (int i = 0; i < 4; ++i) out[i] = small[i];
+        out[4] = R.stamp;
+        out[5] = R.tag;
+        out[6] = R.p;
+        out[7] = R.rounds;
       }
     }
     if (!T.sync()) return false;
-    R.stamp = vload(L.ctr + kStamp);
-    R.tag = vload(L.ctr + kTag);
-    R.p = vload(L.ctr + kParity);
-    R.rounds = vload(L.ctr + kFlipRounds);
+    cnt = out;
+    R.stamp = vload(out + 4);
+    R.tag = vload(out + 5);
+    R.p = vload(out + 6);
+    R.rounds = vload(out + 7);
   }
 }
 
@@ -741,11 +758,16 @@ __global__ void k_all_dirty(Dm M, int nt, int tag, int *D, int *dcnt) {
 // ---------------------------------------------------------------------------
 // The insertion rounds in one launch
 // ---------------------------------------------------------------------------
+#ifdef GQM_HOST_EMU
+constexpr int kLanes = 1;
+#else
+constexpr int kLanes = 32;
+#endif
 // Sum of part[0..nb) before this block's entry, and of all (block-wide).
 CDEV void part_sums(const int *part, int nb, int rank, int *sh, int *before, int *all) {
   if (threadIdx.x < 32) {
     int b = 0, a = 0;
-    for (int r = (int)threadIdx.x; r < nb; r += 32) {
+    for (int r = (int)threadIdx.x; r < nb; r += kLanes) {
       const int v = vload(part + r);
       a += v;
       b += r < rank ? v : 0;
@@ -1564,7 +1586,7 @@ struct Builder {
     launches++;
 #ifdef GQM_HOST_EMU
     (void)blocks;
-    fn(args...);
+    GQM_EMU_GRID(blocks, fn(args...));
     return 0;
 #else
     cudaLaunchConfig_t cfg = {};
@@ -1892,6 +1914,8 @@ int Builder::prepare(int device, int np, const double *pts, int ns, const int *s
     if (cudaMallocHost((void **)&hc, sizeof(int) * kNctr) != cudaSuccess) return GQM_CDT_ERR_MEMORY;
 #ifndef GQM_HOST_EMU
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+#else
+    sms = GQM_EMU_BLOCKS;
 #endif
     dev = device;
   } else if (cudaSetDevice(device) != cudaSuccess) {

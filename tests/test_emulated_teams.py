@@ -9,7 +9,7 @@ import ctypes
 import numpy as np
 import pytest
 
-from gpu_cdt_refine_b200 import inputs, refine
+from gpu_cdt_refine_b200 import cdtio, inputs, refine, triangulate
 from oracle import oracle_py
 
 from test_emulated_kernels import _same, emulated  # noqa: F401  (fixture)
@@ -54,3 +54,15 @@ def test_batch_teams_in_any_order_of_blocks(emulated, order):  # noqa: F811
     assert L.gqm_emu_stuck_count() == 0
     for d, g in zip(doms, got):
         _same(g, oracle_py.refine(d, 20.0, 1, 1)[0])
+
+
+@teams
+@pytest.mark.parametrize("order", [0, 1, 2, 3])
+@pytest.mark.parametrize("points,segments", [(1100, 60), (1100, 0), (4000, 400)])
+def test_triangulation_in_any_order_of_blocks(emulated, order, points, segments):  # noqa: F811
+    pts = inputs.uniform_points(points, 0.0, 1000.0, 7300 + points)
+    seg = inputs.pick_segments(pts, segments, 7301) if segments else np.zeros((0, 2), np.int32)
+    L = _schedule(order)
+    got = triangulate.build_cdt_gpu(pts, seg)
+    assert L.gqm_emu_stuck_count() == 0
+    assert cdtio.same_mesh(inputs.build_cdt(pts, seg), got)
