@@ -66,6 +66,7 @@ struct TeamState {
   int err;
   int job;
   int part[2][kMaxTeam];  // per-block counts of a compaction, by parity
+  int stop[2];            // the error word as a compaction found it, by parity
 };
 // One block's own.
 struct BlockState {
@@ -73,6 +74,7 @@ struct BlockState {
   SmallLists small;
   int cnt[4];
   int wsum[33];
+  int stop;  // a team of one block's ts.stop
 };
 
 #ifdef GQM_CTA_MODE  // the steps as functions of a team
@@ -148,28 +150,32 @@ struct Engine {
   // takes 16 consecutive elements of a tile.  A range of one tile is the lead
   // block's work (one barrier); a longer one is cut into a chunk per block,
   // counted, and emitted behind the counts of the blocks before (two).
-  // Returns GQM_OK or the barrier's failure.
+  // Returns GQM_OK, the barrier's failure, or the error that a step before it
+  // has recorded: every loop of the refinement compacts in each of its rounds,
+  // and none goes on with a mesh that was found inconsistent.
   template <class F, class Mp>
   __device__ __noinline__ int compact(F f, Mp m, int lo, int hi, int *out, int *count) {
 #ifdef GQM_HOST_EMU
-    int *part = ts.part[parity];
+    int *part = ts.part[parity], *stop = ts.stop + parity;
     parity ^= 1;
     if (T.rank == 0) {
+      *stop = ts.err;
       part[0] = 0;
       for (int i = lo; i < hi; ++i)
         if (f(i)) out[part[0]++] = m(i);
     }
     TSYNC();
     *count = part[0];
-    return GQM_OK;
+    return *stop;
 #else
     constexpr int kItems = 16;
     const int tile = (int)blockDim.x * kItems, n = hi - lo;
     const bool one = T.nb == 1 || n <= tile;
     const int rank = (int)T.rank;
-    int *part = ts.part[parity];
+    int *part = ts.part[parity], *stop = T.nb == 1 ? &sh.stop : ts.stop + parity;
     parity ^= 1;
     int b0 = lo, b1 = hi, base = 0;
+    const int err = T.lead() ? vload(&ts.err) : 0;  // its latency passes under the compaction's own loads
     if (!one) {
       const int chunk = ((n + T.nb - 1) / T.nb + kItems - 1) / kItems * kItems;
       b0 = min(hi, lo + rank * chunk);
@@ -210,6 +216,7 @@ struct Engine {
       *count = sh.wsum[32];
       __syncthreads();
     }
+    if (T.lead()) *stop = err;
     if (!one || rank == 0) {
       const int lane = (int)(threadIdx.x & 31u), warp = (int)(threadIdx.x >> 5), nw = (int)(blockDim.x >> 5);
       for (int t0 = b0; t0 < b1; t0 += tile) {
@@ -248,7 +255,7 @@ struct Engine {
     }
     TSYNC();
     if (one && T.nb > 1) *count = vload(part);
-    return GQM_OK;
+    return vload(stop);
 #endif
   }
   // the device error word, read by every thread before anyone can change it
@@ -534,8 +541,6 @@ struct Engine {
       TSYNC();
       int nbad = 0;
       rc = compact(PBad{S.M.tst}, Ident{}, 0, last_triangle, S.bad, &nbad);
-      if (rc) break;
-      rc = read_err();
       if (rc || nbad == 0) break;
       if (rounds >= max_rounds) {
         rc = GQM_ERR_ROUND_LIMIT;

@@ -911,9 +911,10 @@ __device__ __forceinline__ void delete_point(const Mesh &M, int p) {
 // phase in a small step of the 2,000,000-point refinement).
 __device__ __noinline__ int apply_31(const Mesh &M, int gen, int4 r) {
   const int index = r.x, code = r.y & 15, c0 = claimed(M, gen, index);
-  if (r.z < 0 || r.w < 0) {  // a redundant point on the boundary: no such flip
-  raise_err(M, -5);
-  return r.y;
+  if (r.z < 0 || r.w < 0) {  // a redundant point on the boundary: no such flip, and none in the steps to come
+    raise_err(M, -5);
+    M.tflip[index] = 0;
+    return r.y;
   }
   // 3-1 with the triangles across ori (r.z) and ori + 2 (r.w)
   const int ori = m3(code - 3 + 1), o1 = m3(ori + 1), o2 = m3(ori + 2);
