@@ -651,6 +651,7 @@ struct Refiner {
   long cav_cap = 0;
   FlipLists fl{};         // lists of the flip steps, and their control block (device)
   FlipCtl *fc = nullptr;  // = fl.c, in team
+  unsigned gen_seen = 0;  // the control block's generation after the last run
   TeamState *team = nullptr;  // state of the one-launch refinement
   EngineRun *run_d = nullptr;
   char *bars = nullptr;   // barrier words of the flip loop's launch
@@ -777,6 +778,7 @@ struct Refiner {
     emptyt = bad = imark = ilist = sinks = wl = newidx = tail = nullptr;
     fl = FlipLists{};
     fc = nullptr;
+    gen_seen = 0;
     team = nullptr;
     run_d = nullptr;
     bars = nullptr;
@@ -1442,6 +1444,21 @@ struct Refiner {
     return GQM_OK;
   }
 
+  // Claims are ordered by their generation, and those of earlier runs stay in
+  // the arrays: a generation must not pass the end of its 32 bits.  Long before
+  // it does (a run takes hundreds to thousands of them), the arrays and the
+  // numbering start afresh.  The subsegments' entries are cleared in every run,
+  // so that their epoch may start afresh, too.
+  static constexpr unsigned kGenLimit = 1u << 30;
+  void renew_generations() {
+    static_assert(offsetof(FlipCtl, gen) == 0 && offsetof(FlipCtl, epoch) == sizeof(int), "cleared together");
+    if (gen_seen < kGenLimit) return;
+    cudaMemsetAsync(M.fstamp, 0, sizeof(int) * tphys, st);
+    cudaMemsetAsync(M.fmark, 0xff, sizeof(unsigned long long) * tphys, st);
+    cudaMemsetAsync(M.emap, 0, sizeof(int4) * tphys, st);
+    cudaMemsetAsync(fc, 0, 2 * sizeof(int), st);
+    gen_seen = 0;
+  }
   void grow_buffers(int need) {
     if (need & 1) want_p = 2 * pphys;
     if (need & 2) want_t = 2 * tphys;
@@ -1520,6 +1537,7 @@ struct Refiner {
     unsigned long long fb = 0;
     rc = gqm_fallbacks_cta(&fb, 0, st);  // synchronises
     if (rc) return rc;
+    gen_seen = (unsigned)hf.gen;
     if (hrun.status == GQM_ERR_ARENA) return hrun.need_grow ? GQM_OK : GQM_ERR_MEMORY;  // repeated with larger buffers
     hrun.need_grow = 0;
     M.gc2 = hrun.goodcos2;
@@ -1654,6 +1672,7 @@ struct Refiner {
         buf_gen++;
       }
     }
+    renew_generations();
     cudaEventRecord(ev0, st);
     if (grow_dev(&segs, &segs_cap, (size_t)ns + 1)) return GQM_ERR_MEMORY;
     if (ns) cudaMemcpyAsync(segs, dseg_in, sizeof(int2) * ns, cudaMemcpyDeviceToDevice, st);
@@ -1773,6 +1792,7 @@ struct Refiner {
     stats.learned_used = (long long)hc[5];
     FlipCtl hf;
     cudaMemcpy(&hf, fc, sizeof(hf), cudaMemcpyDeviceToHost);
+    gen_seen = (unsigned)hf.gen;
     stats.flip_steps = hf.steps;
     for (int b = 0; b < kFlipProfileBins; ++b) {
       flip_prof_steps[b] = (long long)hf.prof_steps[b];
@@ -2282,6 +2302,10 @@ const char *gqm_status_string(int s) {
     default: return "unknown status";
   }
 }
+#ifdef GQM_HOST_EMU
+// For the tests: the context as after runs that took so many generations.
+void gqm_emu_set_generation(gqm_context *ctx, unsigned gen) { ctx->r.fc->gen = (int)(ctx->r.gen_seen = gen); }
+#endif
 int gqm_version(void) { return 101; }
 #ifndef GQM_CONTRACTED
 #define GQM_CONTRACTED 0
