@@ -29,7 +29,8 @@ __global__ void __launch_bounds__(NT, 1)
     k_flip_loop(Mesh mesh, FlipLists lists, GridBar *bars, const int *team, int small_limit, int small_team,
                 KTimer *ktm, KTimer *stm) {
   const int nb = min(*team, (int)gridDim.x);  // blocks this refinement uses; the rest leave at once
-  if ((int)blockIdx.x >= nb) return;
+  // a barrier broke in an earlier loop of the run: its counts order nothing any more
+  if ((int)blockIdx.x >= nb || bars[0].broken || bars[1].broken) return;
   __shared__ SmallLists sh;
   __shared__ Mesh M;  // the phases are calls: they read the pointers from shared memory
   __shared__ FlipLists L;

@@ -651,7 +651,7 @@ struct Refiner {
   long cav_cap = 0;
   FlipLists fl{};         // lists of the flip steps, and their control block (device)
   FlipCtl *fc = nullptr;  // = fl.c, in team
-  unsigned gen_seen = 0;  // the control block's generation after the last run
+  unsigned gen_seen = 0;  // the control block's generation after the last run (~0u: not known)
   TeamState *team = nullptr;  // state of the one-launch refinement
   EngineRun *run_d = nullptr;
   char *bars = nullptr;   // barrier words of the flip loop's launch
@@ -1448,7 +1448,9 @@ struct Refiner {
   // the arrays: a generation must not pass the end of its 32 bits.  Long before
   // it does (a run takes hundreds to thousands of them), the arrays and the
   // numbering start afresh.  The subsegments' entries are cleared in every run,
-  // so that their epoch may start afresh, too.
+  // so that their epoch may start afresh, too.  A run that fails may leave claims
+  // of generations that the control block does not count (a flip loop whose
+  // barrier broke has them in registers): the next run starts afresh as well.
   static constexpr unsigned kGenLimit = 1u << 30;
   void renew_generations() {
     static_assert(offsetof(FlipCtl, gen) == 0 && offsetof(FlipCtl, epoch) == sizeof(int), "cleared together");
@@ -1458,6 +1460,11 @@ struct Refiner {
     cudaMemsetAsync(M.emap, 0, sizeof(int4) * tphys, st);
     cudaMemsetAsync(fc, 0, 2 * sizeof(int), st);
     gen_seen = 0;
+  }
+  int run(const gqm_cdt_in *in, bool on_device, const gqm_options *opt) {
+    const int rc = run_attempts(in, on_device, opt);
+    if (rc != GQM_OK) gen_seen = ~0u;
+    return rc;
   }
   void grow_buffers(int need) {
     if (need & 1) want_p = 2 * pphys;
@@ -1571,7 +1578,7 @@ struct Refiner {
   }
 
   // ---- the whole refinement ----
-  int run(const gqm_cdt_in *in, bool on_device, const gqm_options *opt) {
+  int run_attempts(const gqm_cdt_in *in, bool on_device, const gqm_options *opt) {
     NvtxRange nvtx("gqm:refine");
     int rc = setup(opt->device);
     if (rc) return rc;

@@ -35,11 +35,13 @@ struct GqmEmuGrid {
 };
 inline int gqm_emu_order = 0;           // the schedule
 inline int gqm_emu_stuck = 0;           // launches whose blocks could not go on
+inline long long gqm_emu_break = -1;    // waits until a launch's waits are given up (-1: never)
 inline thread_local GqmEmuGrid *gqm_emu_cur = nullptr;
 extern "C" __attribute__((weak)) void gqm_emu_schedule(int order) {
   gqm_emu_order = order;
   gqm_emu_stuck = 0;
 }
+extern "C" __attribute__((weak)) void gqm_emu_break_at(long long wait) { gqm_emu_break = wait; }
 extern "C" __attribute__((weak)) int gqm_emu_stuck_count(void) { return gqm_emu_stuck; }
 
 inline void gqm_emu_next(GqmEmuGrid &g) {
@@ -66,12 +68,13 @@ inline bool gqm_emu_wait(const unsigned long long *word, unsigned long long targ
   GqmEmuGrid &g = *gqm_emu_cur;
   const int me = (int)gqm_emu_block.x;
   std::unique_lock<std::mutex> lock(g.m);
+  if (gqm_emu_break >= 0 && gqm_emu_break-- == 0) g.stuck = true;
   g.blocks[me].word = word;
   g.blocks[me].target = target;
   gqm_emu_next(g);
   g.cv.wait(lock, [&] { return g.running == me; });
   g.blocks[me].word = nullptr;
-  return *word >= target;
+  return !g.stuck && *word >= target;
 }
 template <class F>
 void gqm_emu_launch(int n, F f) {

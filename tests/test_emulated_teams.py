@@ -66,3 +66,30 @@ def test_triangulation_in_any_order_of_blocks(emulated, order, points, segments)
     got = triangulate.build_cdt_gpu(pts, seg)
     assert L.gqm_emu_stuck_count() == 0
     assert cdtio.same_mesh(inputs.build_cdt(pts, seg), got)
+
+
+@teams
+@pytest.mark.parametrize("points", [1500, 3000])  # one launch; the flip loop's own launch
+@pytest.mark.parametrize("wait", [200, 1003, 2506])
+def test_context_recovers_from_a_wait_that_ran_out(emulated, points, wait):  # noqa: F811
+    """The waits of a launch are given up in the middle of a flip loop: that call
+    reports it, and the next on the same context gives the oracle's mesh."""
+    cdt = inputs.plain_small(seed=7500 + points, n=points, nseg=points // 15)
+    want, _ = oracle_py.refine(cdt, 20.0, 1, 1)
+    L = _schedule(2)
+    L.gqm_emu_break_at.argtypes = [ctypes.c_longlong]
+    opt = refine.make_options(20.0, 1, 1)
+    opt.max_rounds = 500  # ends a loop that never does
+    ctx = refine.Context(0)
+    try:
+        ctx.set_tuning(small_limit=-1)  # every step by all blocks
+        L.gqm_emu_break_at(wait)
+        with pytest.raises(refine.RefineError) as e:
+            ctx.run_host(cdt, opt)
+        assert e.value.status == -5
+        for _ in range(2):
+            ctx.run_host(cdt, opt)
+            _same(ctx.result(), want)
+    finally:
+        L.gqm_emu_break_at(-1)
+        ctx.close()
