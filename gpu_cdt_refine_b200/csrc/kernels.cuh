@@ -129,6 +129,25 @@ GQM_KERNEL void k_check_input(const double2 *pts, int np, const int *tri, const 
   if (bad) atomicCAS(err, 0, GQM_ERR_ARGUMENT);
 }
 
+// free slots
+__device__ __forceinline__ void clear_point(const Mesh &M, int i) {
+  M.pts[i] = make_double2(0.0, 0.0);
+  M.ps[i] = PS_DELETED;
+  M.pred[i] = 0;
+}
+__device__ __forceinline__ void clear_tri_flags(const Mesh &M, int t) {
+  M.tsg[t] = make_int4(-1, -1, -1, 0);
+  M.tflip[t] = 0;
+  M.tfo[t] = 0;
+  M.tmark[t] = 0;
+}
+__device__ __forceinline__ void clear_tri(const Mesh &M, int t) {
+  M.tv[t] = make_int4(0, 0, 0, 0);
+  M.tn[t] = make_int4(0, 0, 0, 0);
+  M.tst[t] = 0;
+  clear_tri_flags(M, t);
+}
+
 GQM_KERNEL void k_init_tris(Mesh M, const int *tri, const int *nbr, int nt, int tcap) {
   GS_LOOP(t, tcap) {
     if (t < nt) {
@@ -140,15 +159,10 @@ GQM_KERNEL void k_init_tris(Mesh M, const int *tri, const int *nbr, int nt, int 
       nb.w = 0;
       M.tn[t] = nb;
       M.tst[t] = TS_NOTNULL | TS_CHECK;
+      clear_tri_flags(M, t);
     } else {
-      M.tv[t] = make_int4(0, 0, 0, 0);
-      M.tn[t] = make_int4(0, 0, 0, 0);
-      M.tst[t] = 0;
+      clear_tri(M, t);
     }
-    M.tsg[t] = make_int4(-1, -1, -1, 0);
-    M.tflip[t] = 0;
-    M.tfo[t] = 0;
-    M.tmark[t] = 0;
   }
 }
 
@@ -157,11 +171,10 @@ GQM_KERNEL void k_init_points(Mesh M, const double2 *pts, int np, int pcap) {
     if (i < np) {
       M.pts[i] = pts[i];
       M.ps[i] = 0;
+      M.pred[i] = 0;
     } else {
-      M.pts[i] = make_double2(0.0, 0.0);
-      M.ps[i] = PS_DELETED;
+      clear_point(M, i);
     }
-    M.pred[i] = 0;
   }
 }
 
