@@ -1481,9 +1481,14 @@ struct Refiner {
   // 500 points 4.3 and 2.7 ms, 3,000 points 12.2 and 10.9 ms, 100,000 points
   // 21.2 and 19.3 ms, 500,000 points 33.1 and 32.0 ms, 700,000 points 38.3 and
   // 38.3 ms, 1,000,000 points 52.6 and 54.4 ms.
+  // A launch shape that the engine does not have (several blocks in the small
+  // team, 256 threads at up to 255 registers) runs the graph at every size.
   static constexpr int kOneLaunchTris = GQM_ONE_LAUNCH_TRIS;
   bool one_launch_ok = true;
-  bool one_launch(int nt) const { return one_launch_ok && !explore && !col_feat && nt <= kOneLaunchTris; }
+  bool one_launch(int nt) const {
+    return one_launch_ok && !explore && !col_feat && nt <= kOneLaunchTris && tune.small_cluster == 1 &&
+           tune.check_minb == 2;
+  }
   EngineRun hrun{};
   int run_one_launch(const gqm_options *opt, const double *dpts, const int *dtri, const int *dnbr, int np, int nt,
                      int ns, unsigned hsz) {

@@ -170,9 +170,10 @@ typedef struct {
                               than the input's size asks for) */
   int small_limit;         /* flip steps of at most this many queued triangles are run by the small team
                               (default 256; negative: never) */
-  int small_cluster;       /* blocks of the small team: 1 (default; its lists in shared memory), 8 or 16 */
+  int small_cluster;       /* blocks of the small team: 1 (default; its lists in shared memory), 8 or 16 (of a
+                              refinement by graph, which such a value asks for at every size) */
   int check_blocks_per_sm; /* register budget of the flip loop: 2 = 512 threads per SM at most 128 registers
-                              each (default), 1 = 256 threads at up to 255 */
+                              each (default), 1 = 256 threads at up to 255 (of a refinement by graph, as above) */
 } gqm_tuning;
 /* Set / read a context's launch shape.  Set returns GQM_ERR_ARGUMENT for a
  * value out of range; the context keeps its previous shape then. */

@@ -102,6 +102,8 @@ void gqm_emu_launch(int n, F f) {
   }
   for (auto &t : pool) t.join();
 }
-#define GQM_EMU_BLOCKS 4
+inline int gqm_emu_blocks = 4;  // most blocks of a launch
+extern "C" __attribute__((weak)) void gqm_emu_set_blocks(int n) { gqm_emu_blocks = n; }
+#define GQM_EMU_BLOCKS gqm_emu_blocks
 #define GQM_EMU_GRID(blocks, call) gqm_emu_launch(blocks, [&] { call; })
 #define GQM_EMU_WAIT(word, target) gqm_emu_wait(word, target)

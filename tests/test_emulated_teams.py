@@ -47,6 +47,25 @@ def test_flip_loop_in_any_order_of_blocks(emulated, order, points, shape):  # no
 
 @teams
 @pytest.mark.parametrize("order", [0, 1, 2])
+@pytest.mark.parametrize("limit", [40, 300])
+def test_small_team_of_some_of_the_blocks(emulated, order, limit):  # noqa: F811
+    cdt = inputs.plain_small(seed=7150, n=1500, nseg=100)
+    L = _schedule(order)
+    L.gqm_emu_set_blocks(12)
+    ctx = refine.Context(0)
+    try:
+        ctx.set_tuning(small_cluster=8, small_limit=limit)
+        ctx.run_host(cdt, refine.make_options(20.0, 1, 1))
+        got = ctx.result()
+    finally:
+        L.gqm_emu_set_blocks(4)
+        ctx.close()
+    assert L.gqm_emu_stuck_count() == 0
+    _same(got, oracle_py.refine(cdt, 20.0, 1, 1)[0])
+
+
+@teams
+@pytest.mark.parametrize("order", [0, 1, 2])
 def test_batch_teams_in_any_order_of_blocks(emulated, order):  # noqa: F811
     doms = [inputs.plain_small(seed=7200 + i, n=n, nseg=n // 15) for i, n in enumerate([900, 300])]
     L = _schedule(order)
