@@ -2034,12 +2034,14 @@ int gqm_context_autotune(gqm_context *ctx, const gqm_cdt_in *in, int in_on_devic
   double best = 0.0;
   rc = time_of(&best);
   if (rc) return rc;
-  // one field at a time, in order of expected effect; each candidate that the
-  // device cannot run (a cluster size it cannot place) is skipped
+  // one field at a time, in order of expected effect; a candidate that would
+  // launch the same as the shape it is compared with is not timed: the clock's
+  // noise would decide
+  const int most = R.loop_blocks[2];
   const int checks[] = {2, 1};
   const int clusters[] = {1, 8, 16};
   const int limits[] = {128, 256, 512, 1024};
-  const int grids[] = {148 * 2, 148 * 4, 148 * 8};
+  const int grids[] = {most / 2, most / 4, gqm::Refiner::Tuning().step_grid};
   for (int field = 0; field < 4; ++field) {
     const int *vals = field == 0 ? checks : field == 1 ? clusters : field == 2 ? limits : grids;
     const int nv = field == 0 ? 2 : field == 1 ? 3 : field == 2 ? 4 : 3;
@@ -2047,21 +2049,24 @@ int gqm_context_autotune(gqm_context *ctx, const gqm_cdt_in *in, int in_on_devic
       gqm_tuning cand = cur;
       int *f = field == 0 ? &cand.check_blocks_per_sm
                           : field == 1 ? &cand.small_cluster : field == 2 ? &cand.small_limit : &cand.step_grid;
-      if (*f == vals[k]) continue;
+      if (*f == vals[k] || vals[k] < 1) continue;
       *f = vals[k];
+      const int blocks = R.team_blocks(in->numberoftriangles);
       if (gqm_context_set_tuning(ctx, &cand) != GQM_OK) continue;
+      if (field == 3 && R.team_blocks(in->numberoftriangles) == blocks) {
+        gqm_context_set_tuning(ctx, &cur);
+        continue;
+      }
       double ms = 0.0;
       rc = time_of(&ms);
-      if (rc) {
-        gqm_context_set_tuning(ctx, &cur);
-        return rc;
-      }
+      gqm_context_set_tuning(ctx, &cur);
+      if (rc) return rc;
       if (ms < best) {
         best = ms;
         cur = cand;
+        gqm_context_set_tuning(ctx, &cur);
       }
     }
-    gqm_context_set_tuning(ctx, &cur);
   }
   gqm_context_get_tuning(ctx, chosen);
   if (best_ms) *best_ms = best;

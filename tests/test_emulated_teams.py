@@ -112,3 +112,22 @@ def test_context_recovers_from_a_wait_that_ran_out(emulated, points, wait):  # n
     finally:
         L.gqm_emu_break_at(-1)
         ctx.close()
+
+
+@teams
+def test_autotune_chooses_among_launches_that_differ(emulated):  # noqa: F811
+    """Two and one of four blocks are tried beside all four; an input that one
+    block refines has nothing to choose there (six runs: no clock's noise does)."""
+    _schedule(2)
+    opt = refine.make_options(20.0, 1, 1)
+    for points, grids in ((1500, (592, 2, 1)), (300, (592,))):
+        cdt = inputs.plain_small(seed=7550, n=points, nseg=points // 15)
+        for _ in range(6):
+            ctx = refine.Context(0)
+            try:
+                chosen, _ = ctx.autotune(cdt, opt)
+                assert chosen["step_grid"] in grids and chosen == ctx.tuning()
+                ctx.run_host(cdt, opt)
+                _same(ctx.result(), oracle_py.refine(cdt, 20.0, 1, 1)[0])
+            finally:
+                ctx.close()
