@@ -70,7 +70,8 @@ def _cuda_jobs(force=False, extra=None, variant="separate"):
     lib, fmad, objsub = VARIANTS[variant]
     out = os.path.join(HERE, lib)
     hdr = [os.path.join(INC, "gqm_refine.h"), os.path.join(INC, "gqm_triangulateio.h"),
-           os.path.join(CSRC, "predicates.h"), os.path.join(CSRC, "host_copy.h")]
+           os.path.join(CSRC, "predicates.h"), os.path.join(CSRC, "host_copy.h"),
+           os.path.join(CSRC, "sm_share.h")]
     refiner = [os.path.join(CSRC, f) for f in ("kernels.cuh", "gqm_device.cuh", "learned.cuh", "engine.cuh",
                                                   "team.cuh")]
     units = {  # translation unit -> (the headers it includes, its own flags)
@@ -79,7 +80,8 @@ def _cuda_jobs(force=False, extra=None, variant="separate"):
         "flipcl.cu": (hdr + refiner, []),
         "learned.cu": (hdr + [os.path.join(CSRC, "learned.cuh"), os.path.join(CSRC, "team.cuh")], []),
         "cdt_gpu.cu": ([os.path.join(INC, "gqm_cdt.h"), os.path.join(CSRC, "predicates.h"),
-                        os.path.join(CSRC, "host_copy.h"), os.path.join(CSRC, "team.cuh")], []),
+                        os.path.join(CSRC, "host_copy.h"), os.path.join(CSRC, "sm_share.h"),
+                        os.path.join(CSRC, "team.cuh")], []),
         "legacy.cpp": (hdr, []),
     }
     base = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",

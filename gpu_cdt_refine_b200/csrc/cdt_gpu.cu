@@ -50,6 +50,7 @@
 #include "gqm_cdt.h"
 #include "host_copy.h"
 #include "predicates.h"
+#include "sm_share.h"
 #include "team.cuh"
 
 namespace gqm_cdt {
@@ -1443,6 +1444,7 @@ struct Builder {
   GridBar *bar = nullptr;
   int *part = nullptr;
   int sms = 148;
+  gqm_share::Ticket share;
   int stamp = 0, tag = 0;
   long long launches = 0;
 
@@ -1579,15 +1581,16 @@ struct Builder {
     if (np <= 1024) return 1;
     return std::min(std::min(sms, kMaxTeam), std::max(16, np / 512));
   }
-  // One cooperative launch; the barrier words start at zero.
+  // One cooperative launch, to its end, and the counters; the barrier words start
+  // at zero.  (About half of a build is host work, copies and ordinary launches.)
   template <class... P, class... A>
-  int launch_team(void (*fn)(P...), int blocks, A... args) {
+  int run_team(void (*fn)(P...), int np, A... args) {
+    const int blocks = share.take(team_blocks(np), std::min(sms, kMaxTeam));
     cudaMemsetAsync(bar, 0, sizeof(GridBar), st);
     launches++;
 #ifdef GQM_HOST_EMU
     (void)blocks;
     GQM_EMU_GRID(blocks, fn(args...));
-    return 0;
 #else
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
@@ -1598,16 +1601,18 @@ struct Builder {
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, fn, args...) == cudaSuccess ? 0 : GQM_CDT_ERR_CUDA;
+    if (cudaLaunchKernelEx(&cfg, fn, args...) != cudaSuccess) return GQM_CDT_ERR_CUDA;
 #endif
+    const int rc = sync_ctr();
+    share.give();
+    return rc;
   }
   // Lawson flips over the dirty list D (count in ctr[kNd], tag `tag`).
   int run_lawson(int np, gqm_cdt_gpu_stats *sts) {
     KL(k_set, 1, 1)(ctr + kNc, 0);
     KL(k_set, 1, 1)(ctr + kNc + 1, 0);
     launches += 2;
-    int rc = launch_team(k_lawson, team_blocks(np), dm(), lists(), stamp, tag);
-    if (rc == 0) rc = sync_ctr();
+    int rc = run_team(k_lawson, np, dm(), lists(), stamp, tag);
     if (rc) return rc;
     stamp = hc[kStamp];
     tag = hc[kTag];
@@ -1753,8 +1758,7 @@ int Builder::build(int np, const double *pts, int ns, const int *segs, gqm_cdt_g
 
   // 2. insertion rounds
   t0 = clk::now();
-  if ((rc = launch_team(k_insert_all, team_blocks(np), M, lists(), npend, ntri, stamp, tag))) return rc;
-  if ((rc = sync_ctr())) return rc;
+  if ((rc = run_team(k_insert_all, np, M, lists(), npend, ntri, stamp, tag))) return rc;
   stamp = hc[kStamp];
   tag = hc[kTag];
   if (sts) {
@@ -1922,7 +1926,9 @@ int Builder::prepare(int device, int np, const double *pts, int ns, const int *s
     return GQM_CDT_ERR_NO_DEVICE;
   }
   if (!pts && np > 0) return last_status = GQM_CDT_ERR_FEW_POINTS;
+  share.open(device, 2.0 * np, 0.5);
   int rc = build(np, pts, ns, segs, stats);
+  share.close();
   last_status = rc;
   if (rc && (rc == GQM_CDT_ERR_CUDA || cudaGetLastError() != cudaSuccess)) release();
   return rc;

@@ -25,6 +25,7 @@
 
 #include "../../include/gqm_refine.h"
 #include "host_copy.h"
+#include "sm_share.h"
 #include "engine.cuh"
 
 // NVTX ranges around the driver's phases (refinement, encroached-subsegment
@@ -1156,7 +1157,8 @@ struct Refiner {
              check_minb == o.check_minb;
     }
   } tune;
-  int sharers = 1;  // contexts that run on the device at the same time: each takes its part of the SMs
+  gqm_share::Ticket *ticket = nullptr;  // a caller's registration of this run (its own otherwise)
+  int loop_grid = 0;               // blocks of the flip loop's launches in this run
   int loop_blocks[3] = {0, 0, 0};  // most resident blocks of the loop's launch, by register budget (0: not asked yet)
 
   // ---- flip-flop (refine.cu:2328-2490) over the triangles flagged since the last loop ----
@@ -1164,9 +1166,7 @@ struct Refiner {
     NvtxRange nvtx("gqm:flip_flop");
     count_launch(1);
     return gqm_flip_loop_launch(&M, sizeof(M), &fl, sizeof(fl), bars, &ds->team, pred_mode,
-                                std::max(1, loop_blocks[tune.check_minb] / sharers), tune.check_minb, tune.small_limit,
-                                tune.small_cluster,
-                                ktm, stm, st);
+                                loop_grid, tune.check_minb, tune.small_limit, tune.small_cluster, ktm, stm, st);
   }
   // Blocks that a refinement uses.  A barrier of several blocks costs several
   // times that of one, and the largest inputs' steps fill every SM: 980
@@ -1177,8 +1177,21 @@ struct Refiner {
   // and 148 (steps of up to 512 triangles by the first block).
   int team_blocks(int nt) const {
     if (nt <= 2048) return 1;
-    const int most = std::min(tune.step_grid, std::max(1, loop_blocks[tune.check_minb] / sharers));
+    const int most = std::min(tune.step_grid, loop_blocks[tune.check_minb]);
     return std::max(1, std::min(most, std::max(16, nt / 512)));
+  }
+  // The blocks that a refinement by graph uses, and the launch that holds them:
+  // the graph is captured for a number of blocks, so those are all, half, a
+  // quarter of the SMs and so on, and what the run does not use leaves at once.
+  int share_loop(int nt) {
+    const int want = team_blocks(nt), most = loop_blocks[tune.check_minb];
+    const int got = ticket ? ticket->take(want, most) : want;
+    loop_grid = most;
+    if (got < want)
+      while (loop_grid > got) loop_grid = std::max(1, loop_grid / 2);
+    else
+      while (loop_grid / 2 >= got) loop_grid /= 2;
+    return std::min(got, loop_grid);
   }
 
   // ---- splitEncsegs (refine.cu:3180-3778) ----
@@ -1328,6 +1341,7 @@ struct Refiner {
     const void *col_feat, *col_tgt, *col_cnt, *mlp_w, *mlp_b;
     unsigned long long col_cap;
     Tuning tune;
+    int loop_grid;
   };
   RefKey ref_key{};  // what the captured graph was built for
   RefKey ref_key_now() const {
@@ -1346,6 +1360,7 @@ struct Refiner {
     k.mlp_b = mlp_b;
     k.col_cap = col_cap;
     k.tune = tune;
+    k.loop_grid = loop_grid;
     return k;
   }
   void drop_ref_graph() {
@@ -1462,7 +1477,14 @@ struct Refiner {
     gen_seen = 0;
   }
   int run(const gqm_cdt_in *in, bool on_device, const gqm_options *opt) {
+    gqm_share::Ticket own;
+    gqm_share::Ticket *const given = ticket;
+    if (!given) {
+      own.open(opt->device, in->numberoftriangles, 1.0);
+      ticket = &own;
+    }
     const int rc = run_attempts(in, on_device, opt);
+    ticket = given;
     if (rc != GQM_OK) gen_seen = ~0u;
     return rc;
   }
@@ -1539,8 +1561,8 @@ struct Refiner {
     cudaMemsetAsync(&team->bar, 0, sizeof(TeamState) - offsetof(TeamState, bar), st);
     KL(k_ctl_reset, 1, 32)(fc, 64 * max_rounds, &team->err);
     gqm_fallbacks_cta(nullptr, 1, st);
-    int rc = gqm_refine_one_launch(&S, sizeof(S), &c, run_d, team, pred_mode, team_blocks(nt), tune.small_limit, ktm,
-                                   stm, st);
+    const int blocks = ticket ? ticket->take(team_blocks(nt), loop_blocks[tune.check_minb]) : team_blocks(nt);
+    int rc = gqm_refine_one_launch(&S, sizeof(S), &c, run_d, team, pred_mode, blocks, tune.small_limit, ktm, stm, st);
     if (rc) return rc;
     cudaEventRecord(ev1, st);
     cudaMemcpyAsync(&hrun, run_d, sizeof(EngineRun), cudaMemcpyDeviceToHost, st);
@@ -1759,7 +1781,7 @@ struct Refiner {
     hds.pointblock = pointblock;
     hds.triblock = triblock;
     hds.max_rounds = max_rounds;
-    hds.team = team_blocks(nt);
+    hds.team = share_loop(nt);
     cudaMemcpyAsync(ds, &hds, sizeof(DState), cudaMemcpyHostToDevice, st);
     rc = run_refinement();
     if (rc == 0) {
@@ -2254,6 +2276,10 @@ int gqm_refine_batch(int ndomains, const gqm_cdt_in *in, gqm_cdt_out *out, const
   for (int i = 0; i < ndomains; ++i) order[i] = i;
   std::stable_sort(order.begin(), order.end(),
                    [&](int a, int b) { return in[a].numberofpoints > in[b].numberofpoints; });
+  // the first domain of every worker is registered before any of them starts
+  std::vector<gqm_share::Ticket> tickets(ndomains);
+  for (int k = 0; k < workers; ++k)
+    tickets[k].open(opt[order[k]].device, in[order[k]].numberoftriangles, 1.0);
   std::atomic<int> next(0), first_err(0), err_dom(-1);
   auto work = [&](int) {
     gqm_context *ctx = nullptr;
@@ -2262,14 +2288,15 @@ int gqm_refine_batch(int ndomains, const gqm_cdt_in *in, gqm_cdt_out *out, const
       if (k >= ndomains || first_err.load() != 0) break;
       int d = order[k];
       int rc = GQM_OK;
-      if (!ctx) {
-        rc = gqm_context_create(opt[d].device, &ctx);
-        // launches that all fit run side by side; each on the whole GPU would
-        // run one after another
-        if (rc == GQM_OK) ctx->r.sharers = workers;
-      }
+      if (!ctx) rc = gqm_context_create(opt[d].device, &ctx);
+      if (k >= workers) tickets[k].open(opt[d].device, in[d].numberoftriangles, 1.0);
       gqm_stats st;
-      if (rc == GQM_OK) rc = gqm_context_run(ctx, &in[d], 0, &opt[d], &st);
+      if (rc == GQM_OK) {
+        ctx->r.ticket = &tickets[k];
+        rc = gqm_context_run(ctx, &in[d], 0, &opt[d], &st);
+        ctx->r.ticket = nullptr;
+      }
+      tickets[k].close();
       if (rc == GQM_OK) rc = gqm_context_result(ctx, &out[d]);
       if (rc == GQM_OK && stats) stats[d] = st;
       if (rc != GQM_OK) {

@@ -76,8 +76,15 @@ inline bool gqm_emu_wait(const unsigned long long *word, unsigned long long targ
   g.blocks[me].word = nullptr;
   return !g.stuck && *word >= target;
 }
+inline int gqm_emu_largest = 0;  // most blocks of a launch since that was last asked
+extern "C" __attribute__((weak)) int gqm_emu_largest_launch(void) {
+  const int n = gqm_emu_largest;
+  gqm_emu_largest = 0;
+  return n;
+}
 template <class F>
 void gqm_emu_launch(int n, F f) {
+  gqm_emu_largest = std::max(gqm_emu_largest, n);
   GqmEmuGrid g;
   g.blocks.resize(n);
   g.rng.seed((unsigned)gqm_emu_order);
