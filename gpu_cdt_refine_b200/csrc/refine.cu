@@ -917,10 +917,12 @@ struct Refiner {
   }
 
   // ---- capacity management ----
+  // delete_point changes a point's status with an atomic on the word it lies in
+  static size_t whole_words(long n) { return ((size_t)n + 3) & ~(size_t)3; }
   int alloc_points(long n) {
     long old = pphys;
     if (n <= old) return GQM_OK;
-    if (regrow(&M.pts, old, n) || regrow(&M.ps, old, n) || regrow(&M.pred, old, n) || regrow(&emptyp, 0, n) ||
+    if (regrow(&M.pts, old, n) || regrow(&M.ps, old, whole_words(n)) || regrow(&M.pred, old, n) || regrow(&emptyp, 0, n) ||
         regrow(&pnew, old, n) || regrow(&tail, 0, std::max<long>(n, tphys)))
       return GQM_ERR_MEMORY;
     // new slots are deleted points
