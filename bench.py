@@ -573,7 +573,7 @@ def run_ours(args, rank, world, local_rank):
                24 * nt_out + 8 * ns_out + 60 * nt_out)
         path_gbs = alg / (ms / 1e3) / 1e9
         top = dict(roofs[0]) if roofs else {}
-        top.update({"timing": "per-launch device timers (%globaltimer, first block start to last block end) in "
+        top.update({"timing": "device timers (%globaltimer, stamped by the launch's lead thread around each phase) in "
                               "one extra probed step after the timed region, on the context's stream",
                     "path_achieved_gbs": path_gbs, "path_frac": path_gbs / peak, "kernels": roofs})
         cfg = config(args, cdt)

@@ -427,12 +427,15 @@ double ms_since(std::chrono::steady_clock::time_point t0) {
 // domain alone.  A domain of n points takes a team of nb blocks about
 // L + P / nb: L = 1.35 log2(n) - 8.8 ms for the chain of its steps (at least
 // 1 ms), whatever the team, and P = 0.75 ms per 1,000 points for the work in
-// them (measured: 49,497 points take 48.6, 32.7, 22.1, 16.8, 14.3 and 13.1 ms
-// with 1, 2, 4, 8, 16 and 32 blocks).  The team size is the one whose queue,
-// largest domain first, ends soonest by that.  Measured for domains of 200 to
-// 50,000 points, one block per team and this rule: 16 domains 53.5 and 16.7 ms,
-// 64 domains 79.8 and 33.5 ms, 256 domains 100.2 and 65.6 ms; 700 domains
-// 115.8 ms with one block and 144.3 ms with two.
+// them (measured on an idle GPU: 49,497 points take 48.6, 32.7, 22.1, 16.8, 14.3
+// and 13.1 ms with 1, 2, 4, 8, 16 and 32 blocks).  The team size is the one whose
+// queue, largest domain first, ends soonest by that.  With all SMs busy the times
+// are 1.6 to 2 times the rule's: it stands for the order of the team sizes, not
+// for the time of a batch (256 domains of 200 to 50,000 points: 49 and 37 ms by
+// the rule with one and two blocks, 100.2 and 65.6 ms measured).  Measured with
+// one block per team and with the rule's choice: 16 domains 53.5 and 16.7 ms, 64
+// domains 79.8 and 33.5 ms, 256 domains 100.2 and 65.6 ms; 700 domains 115.8 ms
+// with one block, the rule's choice, and 144.3 ms with two.
 constexpr int kTeamSizes[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48};
 int blocks_per_team(const gqm_cdt_in *in, const std::vector<int> &ids, long resident) {
   std::vector<double> n;

@@ -566,6 +566,8 @@ struct Engine {
       rc = split_triangles(nbad);
       if (rc == GQM_OK) rc = split_encsegs();
       if (rc) break;
+      // no barrier between this step and the next: k_mark_bad reads other bits of
+      // the status bytes than the one that is cleared here
       k_points_old(S.M, last_point);
       rounds++;
     }

@@ -856,8 +856,8 @@ __device__ __noinline__ void flip_check(const Mesh &M, const int *q, int n, int 
 #else
   // More than two triangles for every four threads: the lanes' repeated loads
   // cost more than the edges one after another (the check phases of the steps
-  // by all blocks of the 2,000,000-point refinement: 17.7 ms with four lanes
-  // throughout, 12.4 ms with this rule; of the 10,000-point one 0.70 and 0.66 ms).
+  // by all blocks of a 2,000,000-point refinement: 17.6 ms with four lanes
+  // throughout, 12.7 ms with this rule; of a 10,000-point one 0.70 ms both ways).
   if (n > size / 2) return flip_check_many<PRED>(M, q, n, gen, L, rec, live, nred, tid, size);
   const int lane = (int)(threadIdx.x & 31u), e = lane & 3, first = lane & 28;
   const int items = size >> 2;

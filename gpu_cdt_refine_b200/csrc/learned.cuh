@@ -91,8 +91,8 @@ __host__ __device__ inline float mlp_forward_row(const MlpDev &P, const float *f
 // ---------------------------------------------------------------------------
 constexpr int kW1Stride = kFeat + 8, kW2Stride = kHid + 8, kXStride = kFeat + 8;
 // warps of a block that run the network: eight in the grid-wide placement
-// kernel; four inside the persistent batch kernel, which keeps its shared
-// memory under 32 KB so that the L1 left to its stack is not cut
+// kernel; four inside the teams' kernels, whose 44 KB of static shared memory
+// leave no room for four more input tiles of 2.5 KB under the 48 KB limit
 #ifdef GQM_CTA_MODE
 constexpr int kInferWarpsMax = 4;
 #else

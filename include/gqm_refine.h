@@ -181,8 +181,8 @@ int gqm_context_set_tuning(gqm_context *ctx, const gqm_tuning *t);
 int gqm_context_get_tuning(gqm_context *ctx, gqm_tuning *t);
 /* Autotuner (no counterpart in the reference): refines `in` (host or device
  * arrays, as gqm_context_run) once per candidate launch shape, one field at a
- * time (check kernel budget, small-step kernel, small-step limit, step grid),
- * keeping each field's fastest value by the device time of the refinement
+ * time (register budget, small team, small-step limit, blocks of a step; shapes
+ * that would launch the same are not timed), keeping each field's fastest value by the device time of the refinement
  * (the best of `repeats` runs, at least 1).  The chosen shape is set on the
  * context and written to *chosen; *best_ms (may be NULL) receives its time.
  * `in` is typically a sample of the workload to be refined; its result is
