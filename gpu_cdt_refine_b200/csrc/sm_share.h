@@ -13,8 +13,8 @@
 // Time of one call with four threads calling, each launch on the whole GPU and
 // with this rule (B200; as launches of one phase each, before: in brackets):
 // refinement of 10,000 points 3.4 and 2.7 ms (6.8), of 100,000 points 22.5 and
-// 7.2 ms (12.6), of 300,000 points 25.7 and 11.0 ms (16.5); triangulation of
-// 200,000 points 4.8 and 2.8 ms (3.6), of 1,000,000 points 12.0 and 10.1 ms (9.4).
+// 7.1 ms (12.6), of 300,000 points 25.7 and 10.8 ms (16.5); triangulation of
+// 200,000 points 4.8 and 2.7 ms (3.6), of 1,000,000 points 12.0 and 9.8 ms (9.4).
 #pragma once
 #include <algorithm>
 #include <mutex>
